@@ -1,0 +1,87 @@
+// Part of libctraj_probes.so (bench_kernels/).  Check of the exact mode's FP64
+// forms (fp64.cuh) against the IEEE operations they stand for, over generated
+// operands: random significands with exponents of the lens pass and of the
+// whole allowed range, significands near all-zeros and all-ones, and operands
+// built to lie next to exact results and rounding boundaries (squares, products
+// and their neighbours).
+#include <cuda_runtime.h>
+
+#include "fp64.cuh"
+
+namespace {
+
+__device__ __forceinline__ unsigned long long mix(unsigned long long x) {  // splitmix64
+  x += 0x9E3779B97F4A7C15ull;
+  x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+  x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+  return x ^ (x >> 31);
+}
+
+// a double in [2^-e, 2^e) with a random or extreme significand
+__device__ __forceinline__ double operand(unsigned long long h, int e, unsigned kind) {
+  unsigned long long sig = mix(h) & 0xFFFFFFFFFFFFFull;
+  if (kind == 1) sig = mix(h) & 0x1F;
+  if (kind == 2) sig = 0xFFFFFFFFFFFFFull - (mix(h) & 0x1F);
+  if (kind == 3) sig &= ~((1ull << (mix(h + 7) % 52)) - 1);
+  const unsigned long long ex = 1023ull - unsigned(e) + mix(h + 1) % unsigned(2 * e);
+  return __longlong_as_double((long long)(ex << 52 | sig));
+}
+__device__ __forceinline__ double nudge(double a, unsigned long long h) {
+  return __longlong_as_double(__double_as_longlong(a) + (long long)(h % 5) - 2);
+}
+__device__ __forceinline__ bool same(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+
+__global__ void k_fp64_check(const long long n, const unsigned long long seed, unsigned long long* bad) {
+  unsigned long long b_sqrt = 0, b_div = 0, b_div6 = 0, unsure = 0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    const unsigned long long h = mix(seed * 0x100000001ull + (unsigned long long)k);
+    const unsigned kind = unsigned(h & 7);
+    const int e = (h >> 3 & 3) ? 60 : 190;
+    const double a = operand(h, e, kind), b = operand(h + 100, e, unsigned(h >> 5 & 7));
+    // a square root and quotients by it, as the lens force forms them
+    double x = a;
+    if (kind == 4) x = nudge(__dmul_rn(a, a), h >> 9);
+    double hh;
+    bool sure;
+    const double r = ctraj::sqrt64(x, hh, sure);
+    b_sqrt += !sure || same(r, __dsqrt_rn(x)) ? 0 : 1;
+    unsure += kind > 0 || sure ? 0 : 1;
+    double num = b;
+    if (kind == 5) num = nudge(__dmul_rn(b, r), h >> 9);
+    if (kind == 6) num = -num;
+    if (kind == 7) num = (h >> 12 & 1) ? 0.0 : -0.0;
+    if (sure) {  // r is the rounded root
+      const double v = ctraj::div64(num, r, ctraj::scale2(hh, 1), sure);
+      b_div += !sure || same(v, __ddiv_rn(num, r)) ? 0 : 1;
+      unsure += kind > 0 || sure ? 0 : 1;
+    }
+    // by a divisor whose rounded reciprocal is given
+    if (kind == 5) num = nudge(__dmul_rn(b, a), h >> 9);
+    const double v = ctraj::div64(num, a, __ddiv_rn(1.0, a), sure);
+    b_div += !sure || same(v, __ddiv_rn(num, a)) ? 0 : 1;
+    unsure += kind > 0 || sure ? 0 : 1;
+    num = kind == 5 ? nudge(__dmul_rn(6.0, b), h >> 9) : kind == 7 ? -0.0 : num;
+    if (ctraj::div6_ok(num)) b_div6 += same(ctraj::div6(num), __ddiv_rn(num, 6.0)) ? 0 : 1;
+  }
+  if (b_sqrt) atomicAdd(bad, b_sqrt);
+  if (b_div) atomicAdd(bad + 1, b_div);
+  if (b_div6) atomicAdd(bad + 2, b_div6);
+  if (unsure) atomicAdd(bad + 3, unsure);
+}
+
+}  // namespace
+
+// Returns 0 and, of n generated operand sets, the number of square roots,
+// quotients and quotients by 6 that differ from the IEEE operation without
+// saying so, and how many of the random ones (an eighth of the sets, three
+// operations each) were unsure.
+extern "C" int ctraj_peak_fp64_check(long long n, unsigned long long seed, unsigned long long* mismatches) {
+  if (n < 1 || !mismatches) return -1;
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, 4 * sizeof *d) != cudaSuccess) return -3;
+  cudaMemset(d, 0, 4 * sizeof *d);
+  k_fp64_check<<<1216, 256>>>(n, seed, d);
+  cudaError_t e = cudaMemcpy(mismatches, d, 4 * sizeof *d, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : -2;
+}

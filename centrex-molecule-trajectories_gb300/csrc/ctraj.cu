@@ -507,8 +507,15 @@ int launch_all(ctraj_context* c, const Plan& P, const RunDev& R0, Queue* q, int*
       out.count = c->chunk_ctl.as<unsigned>(k * kCtlWords * sizeof(unsigned));
       out.max_steps = out.count + 1;
       out.head = out.count + 2;
-      kl<<<grid, kLensThreads, smem, s>>>(P, R, i, in, out, q[nxt], lens_chunks[k], la);
-      CT_CUDA(cudaGetLastError());
+      bool launched = false;
+      if constexpr (k64) {
+        const int st = launch_chunk64(c, kOut, P, R, i, in, out, q[nxt], count, lens_chunks[k], &launched);
+        if (st) return st;
+      }
+      if (!launched) {
+        kl<<<grid, kLensThreads, smem, s>>>(P, R, i, in, out, q[nxt], lens_chunks[k], la);
+        CT_CUDA(cudaGetLastError());
+      }
       ++*launches;
       in = out;
       std::swap(cur, alt);
@@ -588,7 +595,10 @@ int ctraj_destroy(ctraj_context* c) {
   if (!c) return CTRAJ_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  for (auto& t : c->tables) t.dev.release();
+  for (auto& t : c->tables) {
+    t.dev.release();
+    t.rec64.release();
+  }
   c->lens_tables.release();
   for (auto& q : c->queue) q.release();
   c->qctl.release();
@@ -776,6 +786,7 @@ int ctraj_set_force_table(ctraj_context* c, int32_t id, const ctraj_force_table*
   if (t->kind == CTRAJ_TABLE_STARK_SPLINE) ht.coef.assign(t->coef, t->coef + size_t(t->n_knots - 1) * 4);
   else ht.values.assign(t->values, t->values + t->n_knots);
   ht.uploaded = false;
+  ht.rec64_built = false;
   c->lens_tables_dirty = true;
   ++c->generation;
   return CTRAJ_OK;
@@ -1130,6 +1141,7 @@ static int batch_peer(ctraj_context* c) {
       p->tables[t].coef = c->tables[t].coef;
       p->tables[t].values = c->tables[t].values;
       p->tables[t].uploaded = false;
+      p->tables[t].rec64_built = false;
     }
     p->lens_tables_dirty = true;
     p->chunk = c->chunk;

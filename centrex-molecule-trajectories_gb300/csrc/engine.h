@@ -71,6 +71,8 @@ struct HostTable {
   std::vector<double> knots, coef, values;
   DevBuf dev;  // knots | coef | values
   bool uploaded = false;
+  DevBuf rec64;  // the exact-mode lens kernel's records (launch_chunk64), built on its first use
+  bool rec64_built = false, rec64_ok = false;
 };
 
 
@@ -227,6 +229,12 @@ using LensKernel = void (*)(const Plan, const RunDev, const int, const Queue, co
                             const LensArgs);
 LensKernel lens_kernel(bool k64, bool out, bool ring, int force, bool staged);
 LensKernel sweep_lens_kernel(int force, bool staged);
+
+// One chunk of the exact-mode (FP64) lens pass through k_lens_chunk64
+// (k_chunk64.cu) for a queue of at most `count` molecules; *launched stays
+// false when the lens or its table does not fit it (k_lens_chunk then).
+int launch_chunk64(ctraj_context* c, bool out, const Plan& P, const RunDev& R, int li, const Queue& Qin,
+                   const Queue& Qcont, const Queue& Qnext, unsigned count, int chunk, bool* launched);
 
 // The persistent FP32 lens kernel (k_persist.cu) for force law `force`, mode
 // kMode* (plain, ring, batch), staged table or not; lanes: molecules per CTA
