@@ -1,4 +1,6 @@
-// Part of libctraj_probes.so (bench_kernels/).  Check of the exact mode's FP64
+// Part of libctraj_probes.so (bench_kernels/).  Checks of the square roots and
+// quotients the kernels form themselves.  The lens pass's FP32 root (sqrt32)
+// against sqrtf for every float of its range; the exact mode's FP64
 // forms (fp64.cuh) against the IEEE operations they stand for, over generated
 // operands: random significands with exponents of the lens pass and of the
 // whole allowed range, significands near all-zeros and all-ones, and operands
@@ -7,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "fp64.cuh"
+#include "molecule.cuh"
 
 namespace {
 
@@ -69,7 +72,30 @@ __global__ void k_fp64_check(const long long n, const unsigned long long seed, u
   if (unsure) atomicAdd(bad + 3, unsure);
 }
 
+// every float of [2^-100, 2^100), and 0
+__global__ void k_sqrt32_check(unsigned long long* bad) {
+  unsigned long long b = 0;
+  const unsigned lo = unsigned(127 - 100) << 23, hi = unsigned(127 + 100) << 23;
+  for (unsigned k = lo + blockIdx.x * blockDim.x + threadIdx.x; k < hi; k += gridDim.x * blockDim.x) {
+    const float a = __uint_as_float(k);
+    b += __float_as_uint(ctraj::sqrt32(a)) == __float_as_uint(sqrtf(a)) && ctraj::sqrt32_ok(a) ? 0 : 1;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) b += __float_as_uint(ctraj::sqrt32(0.0f)) != 0u || !ctraj::sqrt32_ok(0.0f);
+  if (b) atomicAdd(bad, b);
+}
+
 }  // namespace
+
+extern "C" int ctraj_peak_sqrt32_check(unsigned long long* mismatches) {
+  if (!mismatches) return -1;
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, sizeof *d) != cudaSuccess) return -3;
+  cudaMemset(d, 0, sizeof *d);
+  k_sqrt32_check<<<1216, 256>>>(d);
+  cudaError_t e = cudaMemcpy(mismatches, d, sizeof *d, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : -2;
+}
 
 // Returns 0 and, of n generated operand sets, the number of square roots,
 // quotients and quotients by 6 that differ from the IEEE operation without

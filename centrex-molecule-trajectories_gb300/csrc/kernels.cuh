@@ -815,7 +815,8 @@ static __global__ void __launch_bounds__(kOrderThreads) k_order_place(const __gr
 // the queue in `order`, so lanes stay busy while work remains.
 // Phase B (queue empty): every `interval` steps the CTA counts its molecules
 // and, when they fit in fewer warps, moves them through shared memory into
-// the lowest warps.  The emptied warps wait at the barrier without issuing,
+// a few per scheduler (spread_warps).  The emptied warps wait at the barrier
+// without issuing,
 // so the last, longest-lived molecules run with little contention for the
 // SM's issue slots -- their step time approaches the latency of one RK4 step.
 //
@@ -834,6 +835,24 @@ struct SwapSlot {
 
 constexpr int kPersistThreads = 512;
 constexpr int kPersistService = 64;  // default steps between phase-A services
+// Steps between looks at a molecule (persist_pass).  A look costs about 170
+// cycles: the next group starts after the last step's radius and the branch on
+// it.  1e6 molecules in the focusing lens (28 per warp): 631 us with groups of
+// 4, 593 with 8, 630 with 16 (longer groups are done again more often); 1e4 (1
+// or 2 per warp): 425, 400, 382.
+constexpr int kRunGroup = 8;
+static_assert(64 % kRunGroup == 0, "groups fill 64 steps");
+// Phase B loads table pieces ahead while a CTA's molecules fill at most this
+// many warps: 176-212 cycles per step at one warp per scheduler against 229-264,
+// but 39.6 against 33.6 cycles per warp and step at four.
+constexpr unsigned kSparseWarps = 4;
+// Warps that n molecules of a CTA are spread over: four (one per scheduler) or
+// a multiple of it, as few as hold them.  Thin warps step faster than packed
+// ones: fewer bank conflicts, missed pieces and ends per warp.
+template <int kT>
+__device__ __forceinline__ unsigned spread_warps(unsigned n) {
+  return min(unsigned(kT / 32), 4u * ((n + 127u) / 128u));
+}
 
 struct PersistAcc {
   unsigned long long steps = 0, lsteps = 0, band = 0, bad = 0, range = 0, rerr = 0;
@@ -931,8 +950,9 @@ __device__ __forceinline__ void lens_finish(const Plan& P, const RunDev& R, cons
   }
 }
 
-// lens_finish as a call of its own, for the batched sweep's pass: a sweep ends
-// in the pass only the molecules beyond its end records, and inlined there
+// lens_finish as a call of its own, for the passes whose ends are deferred: a
+// plain run ends in the pass no molecule (the allocation-free entry point all),
+// a sweep only the molecules beyond its end records, and inlined there
 // the end's code set the pass's register count (126 at 512 threads, spills
 // at 768 and 1024); called, it costs a stack frame on that cold path and the
 // pass fits 79 registers at 768 threads (lens pass of the bench's sweep 17.3
@@ -1066,16 +1086,121 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     if (lost) x.phase = kLost;
     else if (x.st.n_done == x.st.n_total) x.phase = kExit;
   };
-  auto run = [&](int n_steps) {
+  // `n_steps` steps of the warp's molecules.  With one molecule per thread they
+  // go in groups without a look at the molecule in between (the bore test, the
+  // step count and their branch otherwise sit on the step-to-step dependency
+  // chain: 229 instead of 260-290 cycles per step of a warp alone); a group in
+  // which the molecule ended is done again from its start, step by step.
+  // sparse: few warps of the CTA have molecules, so the step's latency counts
+  // and pieces are loaded ahead (lens_step_ahead), a group with a missed piece
+  // being done again as well; a warp that misses in more than half of its
+  // groups goes on without.  At 1024 threads (64 registers, 32 warps to hide
+  // latency) the linear form steps singly where the lens loses most molecules
+  // and groups are often done again: 8 runs of 3e6 molecules in the focusing
+  // lens 4.39 ms in groups, 4.89 singly; 20 runs of 1e7 in the defocusing one
+  // 13.20 and 13.13.
+  auto run = [&](const int n_steps, const bool sparse) {
     bool any = false;
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) any = any || X[s].phase == kRun;
     if (!__any_sync(kFull, any)) return;
-#pragma unroll 2  // half the loop's own compare and branch per step: 2-4 % on the pass
-    for (int k = 0; k < n_steps; ++k) {
+    int k = 0;
+    if constexpr (kMPT == 1) {
+      PersistSlot<M>& x = X[0];
+      const float b = kSweep ? x.beta : L.beta;
+      // a group's steps by `advance` (true: all of them are the molecule's own)
+      auto group = [&](auto&& advance) {
+        constexpr int n = kRunGroup;
+        const float4 sa = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy), sb = make_float4(x.m.cx, x.m.cy, x.m.cvx, x.m.cvy);
+        bool ok = x.st.n_done + n <= x.st.n_total;
+        if constexpr (kRing) ok = ok && (!rec_on || x.to_rec > n);
+        if (ok) ok = advance();
+        if (ok) {
+          x.st.n_done += n;
+          if constexpr (kRing) x.to_rec -= n;
+          if (x.st.n_done == x.st.n_total) x.phase = kExit;
+        } else {
+          x.m.x = sa.x;
+          x.m.y = sa.y;
+          x.m.vx = sa.z;
+          x.m.vy = sa.w;
+          x.m.cx = sb.x;
+          x.m.cy = sb.y;
+          x.m.cvx = sb.z;
+          x.m.cvy = sb.w;
+#pragma unroll 1
+          for (int j = 0; j < n; ++j)
+            if (x.phase == kRun) step(x);
+        }
+      };
+      // largest squared radius of the group within the bore; its distance is
+      // the smallest of the group's, rounding being monotone
+      auto inside = [&](const float r2max) {
+        if (!(r2max <= L.bore2)) return false;
+        if constexpr (kOut) {
+          const float d = __fadd_rn(sqrtf(r2max), -L.bore);
+          if (d > 0.0f) return false;
+          x.m.note(d);
+        }
+        return true;
+      };
+      const PairTable T = pair_table<F>(L, kStaged ? s_tab : L.q);
+      if constexpr (F == kForceStark2Lin && kStaged) {
+        if (sparse) {
+          LinAhead q;
+          q.clear();
+          unsigned missed = 0;
+          for (; k + kRunGroup <= n_steps; k += kRunGroup) {
+            if (k % 64 == 0) {
+              if (!__any_sync(kFull, x.phase == kRun)) return;
+              if (__any_sync(kFull, missed > 64u / (2u * kRunGroup))) break;  // steps too wide to extrapolate
+              missed = 0;
+            }
+            if (x.phase == kRun)
+              group([&]() {
+                float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+                unsigned bad = 0;
 #pragma unroll
-      for (int s = 0; s < kMPT; ++s)
-        if (X[s].phase == kRun) step(X[s]);
+                for (int j = 0; j < kRunGroup; ++j) {
+                  x.m.template lens_step_ahead<kSweep>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, q, r2, bad, b, x.kappa);
+                  r2max = fmaxf(r2max, r2);
+                }
+                missed += bad < 0x3f800000u ? 0u : 1u;
+                return bad < 0x3f800000u && inside(r2max);
+              });
+          }
+        }
+      }
+      if (kT < 1024 || F != kForceStark2Lin || !L.outward) {
+        for (; k + kRunGroup <= n_steps; k += kRunGroup) {
+          if (k % 64 == 0 && !__any_sync(kFull, x.phase == kRun)) return;
+          if (x.phase == kRun)
+            group([&]() {
+              float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+              unsigned flags = 0;
+#pragma unroll
+              for (int j = 0; j < kRunGroup; ++j) {
+                x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
+                                                                      x.kappa);
+                r2max = fmaxf(r2max, r2);
+              }
+              return flags == 0 && inside(r2max);
+            });
+        }
+      }
+    }
+    while (k < n_steps) {
+      const int stop = min(n_steps, k - k % 64 + 64);
+#pragma unroll 2  // half the loop's own compare and branch per step: 2-4 % on the pass
+      for (; k < stop; ++k) {
+#pragma unroll
+        for (int s = 0; s < kMPT; ++s)
+          if (X[s].phase == kRun) step(X[s]);
+      }
+      any = false;
+#pragma unroll
+      for (int s = 0; s < kMPT; ++s) any = any || X[s].phase == kRun;
+      if (!__any_sync(kFull, any)) return;
     }
   };
   // all lanes: the slot-x molecules that were lost or left the lens are
@@ -1108,7 +1233,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         if (!__any_sync(kFull, fin)) return;
       }
     }
-    if constexpr (kMode == kModeSweep) {
+    if constexpr (kMode == kModeSweep || (kMode == kModePlain && !kOut)) {
       lens_finish_call<M, kOut, kMode>(P, R, li, Qin, Qnext, fin, x.m, x.st, x.phase, x.flags, x.idx, x.n0,
                                        x.fresh, x.cfg, S, acc);
       if (fin) x.phase = kIdle;
@@ -1119,15 +1244,27 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     }
   };
 
-  // the first static_entries queue positions, interleaved across CTAs
+  // the first static_entries queue positions, interleaved across CTAs; a queue
+  // shorter than that is dealt out molecule by molecule over the CTAs, each
+  // CTA's share over as few warps per scheduler as hold it
+  const bool short_queue = kMPT == 1 && static_entries > n_in;
+  const unsigned share = blockIdx.x < n_in ? (n_in - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+  unsigned busy = kT / 32u;  // warps with molecules
+  if (short_queue) {
+    busy = spread_warps<kT>(share);
+    const unsigned per = busy ? (share + busy - 1u) / busy : 0u;  // of the CTA's share, in order: a warp's live alike
+    const unsigned j = unsigned(warp) * per + unsigned(lane);
+    if (unsigned(lane) < per && j < share) take(X[0], j * gridDim.x + blockIdx.x);
+  } else {
 #pragma unroll
-  for (int s = 0; s < kMPT; ++s) {
-    const unsigned j = ((unsigned(s) * (kT / 32) + unsigned(warp)) * gridDim.x + blockIdx.x) * 32u + unsigned(lane);
-    if (j < min(n_in, static_entries)) take(X[s], j);
+    for (int s = 0; s < kMPT; ++s) {
+      const unsigned j = ((unsigned(s) * (kT / 32) + unsigned(warp)) * gridDim.x + blockIdx.x) * 32u + unsigned(lane);
+      if (j < min(n_in, static_entries)) take(X[s], j);
+    }
   }
   // phase A
   for (bool exhausted = static_entries >= n_in && static_entries > 0; !exhausted;) {
-    run(service);
+    run(service, false);
     unsigned idle[kMPT], n_idle = 0;
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) {
@@ -1150,9 +1287,12 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
       exhausted = static_entries + *(volatile unsigned*)Qin.head >= n_in;
     }
   }
-  // phase B (every warp of the CTA enters it, then the barriers below match)
+  // phase B (every warp of the CTA enters it, then the barriers below match):
+  // with one warp per scheduler there is nothing to compact, so the warps run
+  // to the end of their molecules
   for (;;) {
-    run(interval);
+    const bool last = kMPT == 1 && busy <= 4u;
+    run(last ? CTRAJ_MAX_LENS_STEPS : interval, busy <= kSparseWarps);
     unsigned held = 0;  // molecules this thread holds
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) {
@@ -1179,7 +1319,8 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     }
     __syncthreads();
     if (total == 0) break;
-    if ((total + 32 * kMPT - 1) / (32 * kMPT) < used) {
+    busy = kMPT == 1 ? spread_warps<kT>(total) : (total + 32 * kMPT - 1) / (32 * kMPT);
+    if (busy < used) {
       unsigned r = base + excl;
 #pragma unroll
       for (int s = 0; s < kMPT; ++s) {
@@ -1198,13 +1339,15 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         }
       }
       __syncthreads();
-      // molecule q goes to slot q % kMPT of thread q / kMPT: the lowest warps fill up
+      // kMPT = 1: in order, evenly over `busy` warps; kMPT = 2: molecule q to slot
+      // q % kMPT of thread q / kMPT, the lowest warps fill up
+      const unsigned per = kMPT == 1 ? (total + busy - 1u) / busy : 32u;
 #pragma unroll
       for (int s = 0; s < kMPT; ++s) {
         PersistSlot<M>& x = X[s];
         x.phase = kIdle;
-        const unsigned q = threadIdx.x * kMPT + unsigned(s);
-        if (q < total) {
+        const unsigned q = kMPT == 1 ? unsigned(warp) * per + unsigned(lane) : threadIdx.x * kMPT + unsigned(s);
+        if (q < total && unsigned(lane) < per) {
           const SwapSlot& w = s_swap[q];
           x.m.x = w.a.x;
           x.m.y = w.a.y;
@@ -1257,7 +1400,8 @@ __global__ void __launch_bounds__(kT, 1) k_lens_persist(const __grid_constant__ 
   __shared__ BlockTally S;
   __shared__ unsigned s_wcount[kT / 32];
   SwapSlot* s_swap = reinterpret_cast<SwapSlot*>(s_dyn + (kStaged ? L.n_int : 0));
-  if (*(volatile unsigned*)Qin.count == 0) return;
+  const unsigned n_in = *(volatile unsigned*)Qin.count;
+  if (n_in < L.min_count || n_in > L.max_count) return;
   tally_init(S);
   if (kStaged)
     for (int k = threadIdx.x; k < L.n_int; k += blockDim.x) s_dyn[k] = __ldg(L.q + k);

@@ -214,8 +214,7 @@ __device__ inline int mesh_nearest32(const LensF& L, const ElemF& f, float px, f
 // and infinity land on the clamp.  Bit-identical to the conversions, on
 // FP32 / integer pipes instead of the conversion pipe.  The soft-transmission
 // kernels (4 % faster) and the linear-table lens lookups (one warp's step
-// 323 -> 231 cycles) use it; the quadratic-table lookups keep the
-// conversions, which measured as fast there.
+// 323 -> 231 cycles) use it, the lens lookups in packed form (force_pair).
 // kNonNeg: s is known to be >= 0 or NaN (a linear Stark table starts at
 // |E| = 0 and its coordinate scale is not negative), so max(s, 0) is left
 // out; only a NaN s then takes the last interval instead of the first, and
@@ -230,53 +229,129 @@ __device__ __forceinline__ void table_interval(const float s, const unsigned las
 }
 
 // ---------------------------------------------------------------------------
-// FP32 force: w such that a_perp = w * (x, y)
+// FP32 force: w such that a_perp = w * (x, y), at two points at once
 // ---------------------------------------------------------------------------
-// kStaged: the whole table is in shared memory (s_tab); otherwise it is read
+// A step's force evaluations come in two pairs: the stage-2 point does not
+// depend on the stage-1 force, nor the stage-4 point on the stage-3 force.
+// Each pair's table coordinates, intervals and offsets go through the packed
+// FP32 instructions (two components per instruction, each rounded as the
+// scalar one).
+// kStaged: the whole table is in shared memory (tab); otherwise tab is read
 // from global memory through the read-only cache.  Lookups past the last
 // interval extrapolate it (as scipy CubicSpline does); s < 0 uses interval 0.
 // `beta` is the table-coordinate scale (L.beta, or a molecule's own in a
 // batched sweep where each configuration has its lens voltage).
-// kScaled: beta is a molecule's own (a batched sweep's configuration), not
-// the table's L.beta, which the host checked to be >= 0.
-template <int F, bool kStaged, bool kScaled = false>
-__device__ __forceinline__ float wforce(float px, float py, const LensArgs& L, const float4* s_tab,
-                                        unsigned& flags, const float beta) {
-  const float r2 = __fmaf_rn(py, py, __fmul_rn(px, px));
-  if (F == kForceStark2Lin) {
-    // quarter-interval piece (w, dw): one 8-byte lookup, ~5.4 bank-conflicted
-    // shared-memory wavefronts per warp instead of ~9 for the 16-byte
-    // quadratic entry; s counts pieces, the table holds 2 * n_int of them
-    const float s = __fmaf_rn(beta, r2, -L.s0);
-    // (the interval without the conversion unit: one warp's RK4 step 231
-    // instead of 323 cycles, bit-identical)
-    unsigned i;
-    float u;
-    // s >= 0: the linear form's table starts at |E| = 0 (s0 <= 0) and L.beta >= 0
-    table_interval<!kScaled>(s, unsigned(2 * L.n_int - 1), __int2float_rn(2 * L.n_int - 1), i, u);
-    const float2 q = kStaged ? reinterpret_cast<const float2*>(s_tab)[i]
-                             : __ldg(reinterpret_cast<const float2*>(L.q) + i);
-    return __fmaf_rn(u, q.y, q.x);
-  }
-  float s, r = 0.0f;
-  if (F == kForceStark2) {
-    s = __fmaf_rn(beta, r2, -L.s0);
-  } else {
-    r = sqrtf(r2);
-    s = __fmaf_rn(beta, r, -L.s0);
-    if (F == kForceRadial) flags |= (r > L.r_max) ? 2u : 0u;
-  }
-  const unsigned i = min(__float2uint_rz(s), unsigned(L.n_int - 1));  // negative s -> 0
-  const float u = __fadd_rn(s, -__uint2float_rn(i));
-  const float4 q = kStaged ? s_tab[i] : __ldg(L.q + i);
-  if (F == kForceRadial) {
-    const float a_r = __fmaf_rn(u, q.y, q.x);
-    return r > 0.0f ? __fdividef(a_r, r) : 0.0f;
-  }
-  const float w = __fmaf_rn(u, __fmaf_rn(u, q.z, q.y), q.x);
-  if (F == kForceStark1) return r > 0.0f ? __fdividef(w, r) : 0.0f;
-  return w;
+// The interval is table_interval's; the linear form leaves its max(s, 0) out:
+// the table starts at |E| = 0 and no coordinate scale is negative, so s >= 0
+// or NaN (last piece; u and the force are NaN).
+struct PairTable {
+  const float4* tab;
+  unsigned last;  // last interval (linear form: last of the 2 n_int pieces)
+  float last_f;
+  __device__ __forceinline__ const float2* pieces() const { return reinterpret_cast<const float2*>(tab); }
+};
+template <int F>
+__device__ __forceinline__ PairTable pair_table(const LensArgs& L, const float4* tab) {
+  const int n = F == kForceStark2Lin ? 2 * L.n_int : L.n_int;
+  return PairTable{tab, unsigned(n - 1), float(n - 1)};
 }
+
+__device__ __forceinline__ float2 pack2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+
+// interval of t = 2^23 + s rounded toward -inf
+__device__ __forceinline__ unsigned interval_of(float t, unsigned last) {
+  return __viaddmin_u32(__float_as_uint(t), 0u - 0x4B000000u, last);
+}
+
+// The rounded square root for a in [2^-100, 2^100) or 0, without the slow-path
+// call of sqrtf that keeps a pair's evaluations from overlapping: g + (a - g^2)
+// h from an approximate root g and h = 1 / (2 g) (Markstein 1990), equal to
+// sqrtf for every such a (bench_kernels/fp64_check.cu runs through them all).
+__device__ __forceinline__ float sqrt32(float a) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(a, 0x1p-100f)));
+  const float g = __fmul_rn(a, y);
+  return __fmaf_rn(__fmaf_rn(-g, g, a), __fmul_rn(0.5f, y), g);
+}
+__device__ __forceinline__ bool sqrt32_ok(float a) { return (a >= 0x1p-100f && a < 0x1p100f) || a == 0.0f; }
+
+// Bits of a step's flags: a lookup above a radial table; kFast: a root outside
+// sqrt32's range.
+enum : unsigned { kFlagAbove = 2u, kFlagRoot = 4u };
+
+// w at squared radii r2.  kFast: roots by sqrt32, the step's flags telling
+// when one was out of its range and the step is to be taken again without.
+template <int F, bool kStaged, bool kFast>
+__device__ __forceinline__ float2 force_pair(const LensArgs& L, const PairTable& T, const float2 r2, const float beta,
+                                             unsigned& flags) {
+  const float2 c23 = pack2(8388608.0f, 8388608.0f);
+  float2 r = r2;
+  if constexpr (F == kForceStark1 || F == kForceRadial) {
+    if constexpr (kFast) {
+      r = pack2(sqrt32(r2.x), sqrt32(r2.y));
+      flags |= sqrt32_ok(r2.x) && sqrt32_ok(r2.y) ? 0u : kFlagRoot;
+    } else {
+      r = pack2(sqrtf(r2.x), sqrtf(r2.y));
+    }
+    if (F == kForceRadial) flags |= (r.x > L.r_max || r.y > L.r_max) ? kFlagAbove : 0u;
+  }
+  const float2 s = __ffma2_rn(pack2(beta, beta), r, pack2(-L.s0, -L.s0));
+  const float2 t = __fadd2_rd(F == kForceStark2Lin ? s : pack2(fmaxf(s.x, 0.0f), fmaxf(s.y, 0.0f)), c23);
+  const unsigned i = interval_of(t.x, T.last), j = interval_of(t.y, T.last);
+  const float2 f = __fadd2_rn(t, neg2(c23));
+  const float2 u = __fadd2_rn(s, pack2(-fminf(f.x, T.last_f), -fminf(f.y, T.last_f)));
+  if constexpr (F == kForceStark2Lin) {
+    const float2 a = kStaged ? T.pieces()[i] : __ldg(T.pieces() + i);
+    const float2 b = kStaged ? T.pieces()[j] : __ldg(T.pieces() + j);
+    return pack2(__fmaf_rn(u.x, a.y, a.x), __fmaf_rn(u.y, b.y, b.x));
+  } else {
+    const float4 a = kStaged ? T.tab[i] : __ldg(T.tab + i), b = kStaged ? T.tab[j] : __ldg(T.tab + j);
+    if constexpr (F == kForceRadial) {
+      const float2 w = pack2(__fmaf_rn(u.x, a.y, a.x), __fmaf_rn(u.y, b.y, b.x));
+      return pack2(r.x > 0.0f ? __fdividef(w.x, r.x) : 0.0f, r.y > 0.0f ? __fdividef(w.y, r.y) : 0.0f);
+    }
+    const float2 w = pack2(__fmaf_rn(u.x, __fmaf_rn(u.x, a.z, a.y), a.x), __fmaf_rn(u.y, __fmaf_rn(u.y, b.z, b.y), b.x));
+    if constexpr (F == kForceStark1)
+      return pack2(r.x > 0.0f ? __fdividef(w.x, r.x) : 0.0f, r.y > 0.0f ? __fdividef(w.y, r.y) : 0.0f);
+    return w;
+  }
+}
+
+// Pieces loaded a step ahead of their use (lens_step_ahead; linear form): the
+// table coordinates s of the last step's stages (1, 2) and (4, 3) and their
+// differences d to the step before, and the pieces at the coordinates
+// extrapolated from them, with the pieces' starts k.
+struct LinAhead {
+  float2 s12, d12, s43, d43;
+  float2 k12, k43;
+  float2 e1, e2, e4, e3;
+  __device__ __forceinline__ void clear() {
+    s12 = d12 = s43 = d43 = e1 = e2 = e4 = e3 = pack2(0.0f, 0.0f);
+    k12 = k43 = pack2(-1.0f, -1.0f);  // s - k >= 1: not a piece's offset
+  }
+  // the next coordinates after s, from the last three: 3 s - 3 s' + s'' = s + 2 d - d'
+  static __device__ __forceinline__ float2 next(const float2 s, float2& last, float2& diff) {
+    const float2 d = __fadd2_rn(s, neg2(last)), p = __fadd2_rn(__ffma2_rn(pack2(2.0f, 2.0f), d, s), neg2(diff));
+    last = s;
+    diff = d;
+    return p;
+  }
+  // the pieces at expected coordinates p12, p43 (any value: the index is clamped)
+  __device__ __forceinline__ void load(const PairTable& T, const float2 p12, const float2 p43) {
+    const float2 c = pack2(8388608.0f, 8388608.0f);
+    const float2 t = __fadd2_rd(p12, c), u = __fadd2_rd(p43, c);
+    e1 = T.pieces()[interval_of(t.x, T.last)];
+    e2 = T.pieces()[interval_of(t.y, T.last)];
+    e4 = T.pieces()[interval_of(u.x, T.last)];
+    e3 = T.pieces()[interval_of(u.y, T.last)];
+    const float2 f = __fadd2_rn(t, neg2(c)), g = __fadd2_rn(u, neg2(c));
+    // as unsigned words a negative start is above the last one and is clamped with it
+    auto clamp = [&](float b) { return __uint_as_float(min(__float_as_uint(b), __float_as_uint(T.last_f))); };
+    k12 = pack2(clamp(f.x), clamp(f.y));
+    k43 = pack2(clamp(g.x), clamp(g.y));
+  }
+};
 
 // Per-molecule lens integration parameters (both precisions).
 struct LensStep {
@@ -768,53 +843,53 @@ struct Mol32 {
 
   __device__ double vel_z() const { return double(vz); }
 
-  // kScaled (batched sweeps): the table holds the unscaled polynomial and each
-  // molecule brings its configuration's coordinate scale beta and force scale
-  // kappa; otherwise both come from L (kappa folded into the table).
-  template <int F, bool kStaged, bool kScaled = false>
-  __device__ bool lens_step(const LensArgs& L, const float dt, const float hdt, const float c2,
-                            const float dt6, const float dt26, const float4* s_tab, unsigned& flags,
-                            const float beta = 0.0f, const float kappa = 1.0f) {
-    const float g = L.g;
-    const float b = kScaled ? beta : L.beta;
-    auto force = [&](float px, float py) {
-      const float w = wforce<F, kStaged, kScaled>(px, py, L, s_tab, flags, b);
-      return kScaled ? __fmul_rn(kappa, w) : w;
-    };
-    // The (x, y) pairs go through the packed FP32 instructions of sm_100+
-    // (FFMA2 / FADD2 / FMUL2): per component the same rounding as the scalar
-    // operations, half the instructions.  Increments are formed in full
-    // precision, then added once with the carried rounding error (the lens
-    // defocuses, so uncompensated rounding of x and v grows to micrometres at
-    // the detector).
-    const float2 p = make_float2(x, y), v = make_float2(vx, vy);
-    const float2 Hdt = make_float2(hdt, hdt), Dt = make_float2(dt, dt), G0 = make_float2(0.0f, -g);
-    const float w1 = force(x, y);
-    const float2 l1 = __ffma2_rn(make_float2(w1, w1), p, G0);
-    const float2 k2 = __ffma2_rn(Hdt, l1, v);
-    const float2 p2 = __ffma2_rn(make_float2(c2, c2), v, p);
-    const float w2 = force(p2.x, p2.y);
-    const float2 l2 = __ffma2_rn(make_float2(w2, w2), p2, G0);
-    const float2 k3 = __ffma2_rn(Hdt, l2, v);
-    const float2 p3 = __ffma2_rn(Hdt, k2, p);
-    const float w3 = force(p3.x, p3.y);
-    const float2 l3 = __ffma2_rn(make_float2(w3, w3), p3, G0);
-    const float2 p4 = __ffma2_rn(Dt, k3, p);
-    const float w4 = force(p4.x, p4.y);
-    const float2 l4 = __ffma2_rn(make_float2(w4, w4), p4, G0);
-    const float2 sum = __fadd2_rn(__fadd2_rn(l1, l2), l3);
-    const float2 dx = __ffma2_rn(make_float2(dt26, dt26), sum, __fmul2_rn(Dt, v));
-    const float2 dv = __fmul2_rn(make_float2(dt6, dt6),
-                                 __ffma2_rn(make_float2(2.0f, 2.0f), __fadd2_rn(l2, l3), __fadd2_rn(l1, l4)));
-    // s += inc with the rounding error carried in c, for both pairs (Fast2Sum:
-    // |s| >= |inc + c| holds because one step changes x and v by far less
-    // than their size)
-    auto neg = [](float2 a) { return make_float2(-a.x, -a.y); };
-    float2 cp = make_float2(cx, cy), cv = make_float2(cvx, cvy);
+  // One step, table-coordinate scale beta; kScaled (batched sweeps): the table
+  // holds the unscaled polynomial and the molecule brings its configuration's
+  // force scale kappa.  r2 is the squared radius of (x, y) on entry and of the
+  // new position on return; the molecule is lost when that exceeds bore2.
+  // The stage pairs are packed (a stage per component), the position and
+  // velocity updates by (x, y); per component each operation is the scalar
+  // one.  Increments are formed in full precision, then added once with the
+  // carried rounding error (the lens defocuses, so uncompensated rounding of x
+  // and v grows to micrometres at the detector).  Stages (4, 3) in this order
+  // make l1 + l4 and l2 + l3 one packed addition.
+  // Linear form, run in groups without a bore test in between (persist_pass): a
+  // warp alone on its scheduler takes 229 cycles (292 with (x, y) packed
+  // throughout and the bore tested between steps), 33.6 instead of 35.4 per SM
+  // at 16 warps, 30.3 instead of 32.0 at 32.
+  struct StagePair {
+    float2 X, Y, Lx, Ly;  // stage points and accelerations, one stage per component
+  };
+  __device__ __forceinline__ void pair_begin(const float c2, StagePair& a) const {
+    a.X = pack2(x, __fmaf_rn(c2, vx, x));
+    a.Y = pack2(y, __fmaf_rn(c2, vy, y));
+  }
+  __device__ __forceinline__ void pair_force(const float2 w, const float g, StagePair& a) const {
+    a.Lx = __ffma2_rn(w, a.X, pack2(0.0f, 0.0f));
+    a.Ly = __ffma2_rn(w, a.Y, pack2(-g, -g));
+  }
+  // the points of stages 4 and 3 from the accelerations of stages 1 and 2; their squared radii
+  __device__ __forceinline__ float2 pair_middle(const float dt, const float hdt, const StagePair& a, StagePair& b) const {
+    const float k2x = __fmaf_rn(hdt, a.Lx.x, vx), k2y = __fmaf_rn(hdt, a.Ly.x, vy);
+    const float k3x = __fmaf_rn(hdt, a.Lx.y, vx), k3y = __fmaf_rn(hdt, a.Ly.y, vy);
+    b.X = pack2(__fmaf_rn(dt, k3x, x), __fmaf_rn(hdt, k2x, x));
+    b.Y = pack2(__fmaf_rn(dt, k3y, y), __fmaf_rn(hdt, k2y, y));
+    return __ffma2_rn(b.Y, b.Y, __fmul2_rn(b.X, b.X));
+  }
+  __device__ __forceinline__ void pair_end(const float dt, const float dt6, const float dt26, const StagePair& a,
+                                          const StagePair& b, float& r2) {
+    const float2 p = pack2(x, y), v = pack2(vx, vy);
+    const float2 sum = pack2(__fadd_rn(__fadd_rn(a.Lx.x, a.Lx.y), b.Lx.y), __fadd_rn(__fadd_rn(a.Ly.x, a.Ly.y), b.Ly.y));
+    const float2 dx = __ffma2_rn(pack2(dt26, dt26), sum, __fmul2_rn(pack2(dt, dt), v));
+    const float2 ux = __fadd2_rn(a.Lx, b.Lx), uy = __fadd2_rn(a.Ly, b.Ly);  // (l1 + l4, l2 + l3)
+    const float2 dv = __fmul2_rn(pack2(dt6, dt6), pack2(__fmaf_rn(2.0f, ux.y, ux.x), __fmaf_rn(2.0f, uy.y, uy.x)));
+    // s += inc with the rounding error carried in c (Fast2Sum: |s| >= |inc + c|
+    // holds because one step changes x and v by far less than their size)
+    float2 cp = pack2(cx, cy), cv = pack2(cvx, cvy);
     const float2 d1 = __fadd2_rn(dx, cp), t1 = __fadd2_rn(p, d1);
-    cp = __fadd2_rn(d1, neg(__fadd2_rn(t1, neg(p))));
+    cp = __fadd2_rn(d1, neg2(__fadd2_rn(t1, neg2(p))));
     const float2 d2 = __fadd2_rn(dv, cv), t2 = __fadd2_rn(v, d2);
-    cv = __fadd2_rn(d2, neg(__fadd2_rn(t2, neg(v))));
+    cv = __fadd2_rn(d2, neg2(__fadd2_rn(t2, neg2(v))));
     x = t1.x;
     y = t1.y;
     vx = t2.x;
@@ -823,9 +898,62 @@ struct Mol32 {
     cy = cp.y;
     cvx = cv.x;
     cvy = cv.y;
-    ax = l1.x;
-    ay = l1.y;
-    const float r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
+    ax = a.Lx.x;
+    ay = a.Ly.x;
+    r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
+  }
+  template <int F, bool kStaged, bool kScaled, bool kFast>
+  __device__ __forceinline__ void lens_step_pair(const LensArgs& L, const PairTable& T, const float dt, const float hdt,
+                                                 const float c2, const float dt6, const float dt26, float& r2,
+                                                 unsigned& flags, const float beta, const float kappa) {
+    StagePair a, b;
+    pair_begin(c2, a);
+    const float2 q12 = pack2(r2, __fmaf_rn(a.Y.y, a.Y.y, __fmul_rn(a.X.y, a.X.y)));
+    float2 w = force_pair<F, kStaged, kFast>(L, T, q12, beta, flags);
+    pair_force(kScaled ? __fmul2_rn(pack2(kappa, kappa), w) : w, L.g, a);
+    const float2 q43 = pair_middle(dt, hdt, a, b);
+    w = force_pair<F, kStaged, kFast>(L, T, q43, beta, flags);
+    pair_force(kScaled ? __fmul2_rn(pack2(kappa, kappa), w) : w, L.g, b);
+    pair_end(dt, dt6, dt26, a, b, r2);
+  }
+  // The linear form's step with the pieces in q, loaded during the step before,
+  // so that no lookup waits for its address: 176 cycles for a warp alone.
+  // `bad` collects the offsets in their pieces as unsigned words: one not in
+  // [0, 1) -- at or above 0x3f800000 -- means a piece was not the lookup's and
+  // the state is not the step's (0.02 % of the pieces: the coordinates' rounding
+  // makes the extrapolation uncertain by about 2 ulp.  A fading-memory filter
+  // instead missed a third of that and took as long, for its own instructions).
+  template <bool kScaled>
+  __device__ __forceinline__ void lens_step_ahead(const LensArgs& L, const PairTable& T, const float dt, const float hdt,
+                                                  const float c2, const float dt6, const float dt26, LinAhead& q,
+                                                  float& r2, unsigned& bad, const float beta, const float kappa) {
+    StagePair a, b;
+    pair_begin(c2, a);
+    const float2 B = pack2(beta, beta), S0 = pack2(-L.s0, -L.s0);
+    const float2 s = __ffma2_rn(B, pack2(r2, __fmaf_rn(a.Y.y, a.Y.y, __fmul_rn(a.X.y, a.X.y))), S0);
+    const float2 u = __fadd2_rn(s, neg2(q.k12));
+    float2 w = pack2(__fmaf_rn(u.x, q.e1.y, q.e1.x), __fmaf_rn(u.y, q.e2.y, q.e2.x));
+    pair_force(kScaled ? __fmul2_rn(pack2(kappa, kappa), w) : w, L.g, a);
+    const float2 s4 = __ffma2_rn(B, pair_middle(dt, hdt, a, b), S0);
+    const float2 u4 = __fadd2_rn(s4, neg2(q.k43));
+    w = pack2(__fmaf_rn(u4.x, q.e4.y, q.e4.x), __fmaf_rn(u4.y, q.e3.y, q.e3.x));
+    bad = max(max(bad, max(__float_as_uint(u.x), __float_as_uint(u.y))),
+              max(__float_as_uint(u4.x), __float_as_uint(u4.y)));
+    const float2 p12 = LinAhead::next(s, q.s12, q.d12), p43 = LinAhead::next(s4, q.s43, q.d43);
+    q.load(T, p12, p43);
+    pair_force(kScaled ? __fmul2_rn(pack2(kappa, kappa), w) : w, L.g, b);
+    pair_end(dt, dt6, dt26, a, b, r2);
+  }
+
+  // One step looked at by itself; true when the molecule left the bore.  Without
+  // kScaled the coordinate scale comes from L and kappa is folded into the table.
+  template <int F, bool kStaged, bool kScaled = false>
+  __device__ bool lens_step(const LensArgs& L, const float dt, const float hdt, const float c2,
+                            const float dt6, const float dt26, const float4* s_tab, unsigned& flags,
+                            const float beta = 0.0f, const float kappa = 1.0f) {
+    float r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
+    lens_step_pair<F, kStaged, kScaled, false>(L, pair_table<F>(L, kStaged ? s_tab : L.q), dt, hdt, c2, dt6, dt26, r2,
+                                               flags, kScaled ? beta : L.beta, kappa);
     if (kOut) note(__fadd_rn(sqrtf(r2), -L.bore));
     return r2 > L.bore2;
   }

@@ -47,7 +47,7 @@ struct LensF {
   int outward;      // stark: w >= 0 over the whole table, the force points away from the axis
 };
 
-// The FP32 constants of the one lens a k_lens_chunk launch integrates, passed
+// The FP32 constants of the one lens a lens launch integrates, passed
 // as their own kernel parameter so every use is a fixed-offset constant-bank
 // operand (the Plan's per-element arrays need an indexed load per use).
 struct LensArgs {
@@ -58,6 +58,8 @@ struct LensArgs {
   float bore2;  // (d/2)^2
   float bore;   // d/2
   int classic;
+  int outward;  // LensF::outward
+  unsigned min_count, max_count;  // k_lens_persist: queue sizes this launch takes
 };
 
 // FP64 view of a force table (device pointers).
@@ -99,6 +101,9 @@ __host__ __device__ inline LensArgs lens_args(const Plan& P, int li, bool staged
   a.bore2 = P.ef[li].c[0];
   a.bore = P.ef[li].c[1];
   a.classic = P.el[li].scheme == CTRAJ_RK4_CLASSIC;
+  a.outward = f.outward;
+  a.min_count = 1u;
+  a.max_count = 0xFFFFFFFFu;
   return a;
 }
 

@@ -25,6 +25,16 @@ def test_forms_equal_the_ieee_operations(seed):
     assert bad[3] < 3 * n / 8 * 1e-4  # unsure: near a tie or a power of two, 2^-17 + 2^-19 of random operands each
 
 
+def test_the_fp32_root_is_sqrtf():
+    from bench_kernels.build import build as build_probes
+
+    lib = ctypes.CDLL(str(build_probes()))
+    lib.ctraj_peak_sqrt32_check.argtypes = [ctypes.POINTER(ctypes.c_ulonglong)]
+    bad = ctypes.c_ulonglong(1)
+    assert lib.ctraj_peak_sqrt32_check(ctypes.byref(bad)) == 0
+    assert bad.value == 0
+
+
 def _beamline(table, scheme, dt):
     import ctraj
 
