@@ -142,18 +142,24 @@ class TrajectorySimulator:
         molecules = []
         ids = np.zeros(0, np.int64)
         if want_out:
-            names = res.label_names()
-            ids = np.array([i for i, s in enumerate(names) if s in aoi], dtype=np.int64)
+            # the molecules of interest by counter slot, as arrays: by name, one
+            # Python object per molecule, took 95 of 100 ms for 1e6 molecules
+            wanted = [k for k, name in enumerate(res.labels) if name in aoi] + ([-1] if DETECTED in aoi else [])
+            hit = np.zeros(n, dtype=bool)
+            for k in wanted:
+                hit |= res.label == k
+            ids = np.flatnonzero(hit)
             if ids.size:
                 max_rows = self._max_rows(cb, beamline, res.final[5, ids])
                 traces = eng.record(cb, n, ids, stride=1, max_rows=max_rows, precision=prec,
                                     ics=ics, xdist=xs, vdist=vs, seed=seed, g=g)
-                for i, rows in zip(ids, traces):
-                    m = Molecule(alive=names[i] == DETECTED)
+                for slot, rows in zip(res.label[ids], traces):
+                    name = cb.label_of(int(slot))
+                    m = Molecule(alive=name == DETECTED)
                     m.trajectory = Trajectory.from_rows(rows)
                     m.trajectory.drop_nans()
                     m.trajectory.n = len(m.trajectory.t)
-                    m.set_aperture_hit(names[i])
+                    m.set_aperture_hit(name)
                     molecules.append(m)
         self.counter = Counter()
         self.counter.counter_dict = res.counter_dict()
