@@ -47,6 +47,7 @@
 #pragma once
 #include <type_traits>
 
+#include "fp64.cuh"
 #include "kernels.cuh"
 
 namespace ctraj {
@@ -801,6 +802,166 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens(const __grid_constan
   dropped = warp_sum(dropped);
   entered = warp_sum(entered);
   if ((threadIdx.x & 31) == 0) {
+    if (steps) atomicAdd(&stats[kSoftStatSteps], steps);
+    if (dropped) atomicAdd(&stats[kSoftStatDropped], dropped);
+    if (entered) atomicAdd(&stats[kSoftStatEntered], entered);
+  }
+}
+
+// Steps that k_soft_lens has taken when it drops a molecule of N steps whose log
+// weight is below the floor first at the test of state k (the state before step
+// k; N: after the last): it tests after every 8 steps the states before the
+// previous 8, then the last whole group's, then the last state's.
+__device__ __forceinline__ int soft_dropped_at(int k, int N) {
+  const int groups = N / 8, g = k / 8 + 1;
+  return g < groups ? 8 * (g + 1) : k < 8 * groups ? 8 * groups : N;
+}
+
+// k_soft_lens in FP64 with four lanes per molecule: bit 0 of the lane its
+// component, bit 1 its half (0: stages 1 and 3 and the position's update; 1:
+// stages 2 and 4 and the velocity's), as in k_lens_chunk64.  Bound by the FP64
+// pipe (64 cycles per warp instruction, whatever the number of lanes): the
+// step takes 32 instructions instead of 85, and the bore tests, which do not
+// feed the dynamics, are done four states at a time, a state per lane: 50 to
+// 66 instructions in one lane, 8 to 17 per step here (beyond z = 38, e =
+// exp(-z) < 2^-54 and the log sigmoid and its derivative are -e and e to the
+// last bit).  Every value is k_soft_lens's, the sums in its order.
+// Up to kQuad64Max queued molecules and checkpoint intervals of whole eights;
+// 1e4 molecules (270 queued), gradient: 22.2 -> 7.5 ms.
+template <bool kGrad>
+__global__ void __launch_bounds__(kSoftThreads) k_soft_lens_quad(const __grid_constant__ SoftPlan S, const SoftQueue Q,
+                                                                 const Coef4<double>* __restrict__ table, double* ckpt,
+                                                                 size_t cap, double* __restrict__ contrib,
+                                                                 unsigned long long* stats) {
+  extern __shared__ unsigned char s_raw[];
+  Coef4<double>* s_tab = reinterpret_cast<Coef4<double>*>(s_raw);
+  stage_table(S, table, s_tab);
+  const unsigned n_in = *Q.count;
+  const int lane = threadIdx.x & 31, part = lane & 3, home = lane & ~3;
+  const bool half = part & 2;
+  const double inv_w = S.inv_w, bore = S.bore, floor_ = S.log_floor;
+  const SoftK<double> C(S);
+  const double g = (part & 1) ? -C.g : -0.0;  // a + (-0.0) is a
+  const int K = S.checkpoint;
+  unsigned long long steps = 0, dropped = 0, entered = 0;
+  const unsigned batches = (n_in + 7u) / 8u, warps = gridDim.x * (blockDim.x / 32u);
+  for (unsigned b = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; b < batches; b += warps) {
+    const unsigned slot = b * 8u + unsigned(lane >> 2);
+    const bool have = slot < n_in;
+    const int64_t i = Q.id[have ? slot : 0u];  // lanes beyond the queue repeat a molecule and store nothing
+    SoftMol<double> m;
+    m.init(S, i);
+    m.front(S);
+    const SoftLensSteps<double> L(S, m.vz);
+    const int N = have ? L.N : 0;
+    double X = (part & 1) ? m.y : m.x, V = (part & 1) ? m.vy : m.vx, c = 0.0;
+    const double c34 = half ? L.dt : L.hdt;
+    int below = -1;  // first state whose test leaves the log weight below the floor
+    // w(p) p + (0 or -g) at the points of one stage pair
+    auto force = [&](const double p) {
+      const double o = __shfl_xor_sync(kFull, p, 1);
+      const double px = (part & 1) ? o : p, py = (part & 1) ? p : o;
+      const double s = fma_(C.beta, fma_(py, py, mul_(px, px)), C.neg_s0);
+      const int hi = hi_word(s);
+      unsigned j = hi < 0 ? 0u : hi >= (1050 << 20) ? 0xffffffffu : __float2uint_rz(trunc_float(s));
+      j = min(j, unsigned(C.n_int - 1));
+      const double u = add_(s, -__hiloint2double(0x43300000, int(j)) + 0x1p52);
+      const Coef4<double> q = s_tab[j];
+      return fma_(mul_(C.kappa, fma_(u, fma_(u, q.q2, q.q1), q.q0)), p, g);
+    };
+    for (int n = 0; __any_sync(kFull, n < N && below < 0); n += 4) {
+      if (kGrad && n % K == 0 && n < N && below < 0) {
+        double* o = ckpt + size_t(n / K) * 8 * cap + slot;
+        o[size_t(part) * cap] = half ? V : X;
+        o[size_t(4 + part) * cap] = c;
+      }
+      double qx = 0.0, qy = 0.0;  // this lane's state to test: after step n + part
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const bool run = n + j < N;
+        const double l12 = force(half ? fma_(L.c2, V, X) : X);
+        const double l34 = force(fma_(c34, fma_(L.hdt, l12, V), X));
+        const double m12 = __shfl_xor_sync(kFull, l12, 2), m34 = __shfl_xor_sync(kFull, l34, 2);
+        // halves: (l1 + l2) + l3 -> dt26 (.) + dt v | 2 (l2 + l3) + (l1 + l4) -> dt6 (.)
+        const double a = add_(l12, half ? m34 : m12), e = add_(half ? m12 : a, l34);
+        const double f = fma_(half ? 2.0 : L.dt, half ? a : V, half ? e : -0.0);
+        const double inc = fma_(half ? L.dt6 : L.dt26, half ? f : e, half ? -0.0 : f);
+        const double s0 = half ? V : X, d = add_(inc, c), t = add_(s0, d);
+        const double err = add_(d, -add_(t, -s0));
+        const double o = __shfl_xor_sync(kFull, t, 2);
+        if (run) {
+          X = half ? o : t;
+          V = half ? t : o;
+          c = err;
+        }
+        const double tx = __shfl_sync(kFull, X, home), ty = __shfl_sync(kFull, X, home + 1);
+        if (part == j) {
+          qx = tx;
+          qy = ty;
+        }
+      }
+      // the four states' tests, added in step order
+      const bool use = n + part < N;
+      const double r2 = fma_(qy, qy, mul_(qx, qx));
+      double h;
+      bool sure;
+      double r = sqrt64(r2, h, sure);
+      if (!sure) r = sqrt_(r2);
+      const double z = mul_(add_(bore, -r), inv_w);
+      double ls, dls;
+      if (__all_sync(kFull, !use || (hi_word(z) >= 0x40430000 && hi_word(z) < 0x7ff00000))) {  // 38 <= z < inf
+        dls = exp(-z);
+        ls = -dls;
+      } else {
+        log_sigmoid(z, ls, dls);
+      }
+      const double dr = use ? mul_(dls, inv_w) : 0.0;
+      ls = use ? ls : 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        m.lw = add_(m.lw, __shfl_sync(kFull, ls, home + j));
+        m.d_bore = add_(m.d_bore, __shfl_sync(kFull, dr, home + j));
+        if (below < 0 && n + j < N && !(m.lw >= floor_)) below = n + j + 1;
+      }
+    }
+    const double x = __shfl_sync(kFull, X, home), y = __shfl_sync(kFull, X, home + 1);
+    const double vx = __shfl_sync(kFull, V, home), vy = __shfl_sync(kFull, V, home + 1);
+    const double cx = __shfl_sync(kFull, c, home), cy = __shfl_sync(kFull, c, home + 1);
+    const double cvx = __shfl_sync(kFull, c, home + 2), cvy = __shfl_sync(kFull, c, home + 3);
+    if (!have || part) continue;  // the quad's first lane finishes the molecule
+    ++entered;
+    bool alive = below < 0;
+    double lam[4] = {0.0, 0.0, 0.0, 0.0}, gz = 0.0;
+    if (alive && S.n_post > 0)  // the apertures behind the lens
+      soft_behind(S, add_(x, cx), add_(y, cy), add_(vx, cvx), add_(vy, cvy), m.vz, L.zrel, m.lw, m.d_ap,
+                  kGrad ? lam : nullptr, &gz);
+    steps += unsigned(alive ? N : soft_dropped_at(below, N));
+    if (!(m.lw >= floor_)) alive = false;
+    if (!alive) {
+      ++dropped;
+      continue;
+    }
+    const size_t cnt = size_t(S.count);
+    double* o = contrib + size_t(i - S.first);
+    const double Tw = exp(m.lw);
+    o[0] = Tw;
+    o[(1 + kSoftAperture) * cnt] = Tw * m.d_ap;
+    o[(1 + kSoftBore) * cnt] = Tw * m.d_bore;
+    if (kGrad) {
+      const unsigned k = atomicAdd(Q.bcount, 1u);
+      Q.bid[k] = int32_t(i);
+      Q.bslot[k] = int32_t(slot);
+      if (S.n_post > 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) Q.bpost[size_t(q) * cap + k] = lam[q];
+        Q.bpost[4 * cap + k] = gz;
+      }
+    }
+  }
+  steps = warp_sum(steps);
+  dropped = warp_sum(dropped);
+  entered = warp_sum(entered);
+  if (lane == 0) {
     if (steps) atomicAdd(&stats[kSoftStatSteps], steps);
     if (dropped) atomicAdd(&stats[kSoftStatDropped], dropped);
     if (entered) atomicAdd(&stats[kSoftStatEntered], entered);

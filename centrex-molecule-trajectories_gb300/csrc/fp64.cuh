@@ -31,6 +31,13 @@
 
 namespace ctraj {
 
+// The exact-mode lens passes give a molecule four lanes up to this many
+// molecules in the queue: 1250 warps, two per scheduler, take 75 x 152 cycles a
+// step of k_lens_chunk64, 313 warps of one lane per molecule 197 x 64 (5 100
+// molecules, quads: 18.7 ms; 10 200, one lane while more than this are left: 27
+// ms; 17 000: 40 ms).
+constexpr unsigned kQuad64Max = 10000;
+
 __device__ __forceinline__ int hi_word(double a) { return __double2hiint(a); }
 
 // |a| in [2^(lo), 2^(hi)): biased exponents [1023 + lo, 1023 + hi); false for
@@ -49,6 +56,13 @@ __device__ __forceinline__ double scale2(double a, int k) {
 // a < b and a <= b for non-negative, non-NaN values, on the integer pipe
 __device__ __forceinline__ bool less_pos(double a, double b) {
   return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
+// float nearest below a >= 0 (0 below the normal floats), on the integer pipe
+__device__ __forceinline__ float trunc_float(double a) {
+  const int hi = hi_word(a);
+  const unsigned lo = unsigned(__double2loint(a));
+  return __uint_as_float(hi < (897 << 20) ? 0u : (unsigned(hi - (896 << 20)) << 3) | (lo >> 29));
 }
 
 // Whether q + a b, a correction of a few ulp(q) at most, may lie within 2^-18

@@ -40,12 +40,6 @@ namespace ctraj {
 
 constexpr int kLens64Threads = 256;  // one CTA per SM beside its staged table, two warps per scheduler
 
-// Up to this many molecules in the queue, four lanes per molecule: 1250 warps,
-// two per scheduler, take 75 x 152 cycles a step, 313 warps of one lane per
-// molecule 197 x 64 (5 100 molecules, quads: 18.7 ms; 10 200, one lane while
-// more than this are left: 27 ms; 17 000: 40 ms).
-constexpr unsigned kQuad64Max = 10000;
-
 constexpr size_t kLens64Staged = 200 * 1024;  // bytes of records a CTA stages at most
 
 // Lens constants of k_lens_chunk64 (built by launch_chunk64).
@@ -60,13 +54,6 @@ struct Lens64 {
   float x0, inv_h;     // interval guess
   int n;               // intervals
 };
-
-// float nearest below a >= 0 (0 below the normal floats), on the integer pipe
-__device__ __forceinline__ float trunc_float(double a) {
-  const int hi = hi_word(a);
-  const unsigned lo = unsigned(__double2loint(a));
-  return __uint_as_float(hi < (897 << 20) ? 0u : (unsigned(hi - (896 << 20)) << 3) | (lo >> 29));
-}
 
 // a_r of lens_force64 at radius r; false when the plain path has to decide.
 template <int F>

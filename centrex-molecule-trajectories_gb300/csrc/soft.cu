@@ -188,8 +188,20 @@ int soft_run(ctraj_context* c, const ctraj_soft_args* a, SoftPlan& S, int li, ct
         if ((st = c->soft_seg.ensure(size_t(kSoftSegStride) * cap * size_t(max_seg) * sizeof(T), 25))) return st;
       }
       grid = int((cap + kSoftThreads - 1) / kSoftThreads);
-      kl<<<grid, kSoftThreads, tb, s>>>(S, Q, c->soft_table.as<Coef4<T>>(), c->soft_ckpt.as<T>(), cap, contrib,
-                                         stats);
+      bool quad = false;
+      if constexpr (std::is_same<T, double>::value) {
+        quad = count <= kQuad64Max && S.checkpoint % 8 == 0;
+        if (quad) {
+          auto kq = a->want_grad ? k_soft_lens_quad<true> : k_soft_lens_quad<false>;
+          CT_CUDA(cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tb)));
+          // eight molecules per warp, a warp per CTA while there are SMs
+          kq<<<std::min((count + 7u) / 8u, unsigned(c->sm_count)), kSoftThreads, tb, s>>>(
+              S, Q, c->soft_table.as<Coef4<T>>(), c->soft_ckpt.as<T>(), cap, contrib, stats);
+        }
+      }
+      if (!quad)
+        kl<<<grid, kSoftThreads, tb, s>>>(S, Q, c->soft_table.as<Coef4<T>>(), c->soft_ckpt.as<T>(), cap, contrib,
+                                           stats);
       CT_CUDA(cudaGetLastError());
       ++launches;
       if (a->want_grad) {
