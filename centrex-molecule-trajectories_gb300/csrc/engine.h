@@ -140,6 +140,7 @@ struct ctraj_context {
   uint64_t soft_table_gen = ~uint64_t(0);
   int soft_table_id = -1, soft_table_size = 0;
   double soft_table_f = 1.0;
+  bool soft_table_outward = false;
   unsigned long long* sweep_host = nullptr;  // pinned: per-configuration counts, totals, stats
   size_t sweep_host_words = 0;
   cudaStream_t side[CTRAJ_MAX_TABLES] = {};

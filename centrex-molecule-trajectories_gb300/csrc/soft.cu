@@ -84,6 +84,8 @@ int soft_plan(const ctraj_context* c, const ctraj_soft_args* a, const double* pr
   S.kappa = -2.0 * alpha / mass;
   S.kappa1 = -2.0 * 3.0 / (R * R * R) / mass;
   S.bore = prm[CTRAJ_SOFT_BORE_R];
+  S.bore_f = float(S.bore);
+  S.length_f = float(L.p[7]);
   S.inv_w = 1.0 / a->width;
   S.g = a->g;
   S.log_floor = a->log_floor;
@@ -128,7 +130,16 @@ int soft_run(ctraj_context* c, const ctraj_soft_args* a, SoftPlan& S, int li, ct
     c->soft_table_id = tid;
     c->soft_table_size = int(sizeof(T));
     c->soft_table_f = f;
+    // W'(E) <= 0 throughout (at the intervals' ends, up to 1e-5 of its largest):
+    // the force kappa W' of a V >= 0 points away from the axis
+    bool out = true;
+    for (int j = 0; j < t.n - 1 && out; ++j) {
+      const double* cj = &t.coef[size_t(j) * 4];
+      out = std::max(cj[2], cj[2] + 2.0 * cj[1] * h + 3.0 * cj[0] * h * h) <= 1e-5 * qmax;
+    }
+    c->soft_table_outward = out;
   }
+  S.outward = c->soft_table_outward && S.V >= 0.0;
   S.kappa /= c->soft_table_f;
   S.kappa1 /= c->soft_table_f;
   const int64_t chunk = std::min<int64_t>(std::max<int64_t>(a->n, 1), kSoftChunk);
@@ -142,9 +153,10 @@ int soft_run(ctraj_context* c, const ctraj_soft_args* a, SoftPlan& S, int li, ct
     CT_CUDA(cudaMemcpyAsync(c->ics.p, a->normals, b, cudaMemcpyHostToDevice, s));
     S.normals = c->ics.as<double>();
   }
-  SoftQueue Q{c->soft_queue.as<int32_t>(), c->soft_ctl.as<unsigned>(0), c->soft_ctl.as<unsigned>(4),
+  // control words: queued from the start, from the end (one 64-bit counter), step bound, survivors
+  SoftQueue Q{c->soft_queue.as<int32_t>(), c->soft_ctl.as<unsigned>(0), int(chunk), c->soft_ctl.as<unsigned>(8),
               c->soft_queue.as<int32_t>(size_t(chunk) * 4), c->soft_queue.as<int32_t>(size_t(chunk) * 8),
-              c->soft_ctl.as<unsigned>(8), nullptr};
+              c->soft_ctl.as<unsigned>(12), nullptr};
   unsigned long long* stats = c->soft_ctl.as<unsigned long long>(256);
   double* partial = c->soft_ctl.as<double>(256 + 8 * kSoftStatCount);
   double* contrib = c->soft_contrib.as<double>();
@@ -171,9 +183,9 @@ int soft_run(ctraj_context* c, const ctraj_soft_args* a, SoftPlan& S, int li, ct
     CT_CUDA(cudaGetLastError());
     ++launches;
     if (a->timing) CT_CUDA(cudaEventRecord(c->ev[1], s));
-    CT_CUDA(cudaMemcpyAsync(c->host_max, Q.count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    CT_CUDA(cudaMemcpyAsync(c->host_max, Q.count, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CT_CUDA(cudaStreamSynchronize(s));
-    const unsigned count = c->host_max[0], max_steps = c->host_max[1];
+    const unsigned count = c->host_max[0] + c->host_max[1], max_steps = c->host_max[2];
     out->lens_molecules += int64_t(count);
     if (count > 0) {
       const size_t cap = count;
