@@ -389,6 +389,7 @@ int prepare(ctraj_context* c, const ctraj_run_args* a, Plan& P, RunDev& R) {
   R.ic_mode = a->ic_mode;
   R.xd = a->xdist;
   R.vd = a->vdist;
+  round_distributions(R);
   if (a->ic_mode == CTRAJ_IC_DEVICE_DRAW) {
     const double zd = a->xdist.kind == CTRAJ_DIST_DISC_POSITION ? a->xdist.p[1] : a->xdist.p[2];
     R.gap0f = P.n_el > 0 ? float(P.el[0].z0 - zd) : 0.f;

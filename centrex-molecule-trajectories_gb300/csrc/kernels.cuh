@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_front(const __grid_constan
   if constexpr (M::kScreenable) {
     const ctraj_element& e0 = P.el[0];
     screen = R.ic_mode == CTRAJ_IC_DEVICE_DRAW && R.xd.kind != CTRAJ_DIST_DISC_POSITION &&
-             isfinite(float(R.xd.p[1])) && P.n_el > 0 &&
+             isfinite(R.xf[1]) && P.n_el > 0 &&
              (e0.type == CTRAJ_CIRCULAR_APERTURE || e0.type == CTRAJ_RECTANGULAR_APERTURE);
   }
   if (screen) {
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_sweep_front(const __grid_c
   if constexpr (M::kScreenable) {
     const ctraj_element& e0 = P.el[0];
     screen = R.ic_mode == CTRAJ_IC_DEVICE_DRAW && R.xd.kind != CTRAJ_DIST_DISC_POSITION &&
-             isfinite(float(R.xd.p[1])) && P.n_el > 0 &&
+             isfinite(R.xf[1]) && P.n_el > 0 &&
              (e0.type == CTRAJ_CIRCULAR_APERTURE || e0.type == CTRAJ_RECTANGULAR_APERTURE);
   }
   if (screen) {

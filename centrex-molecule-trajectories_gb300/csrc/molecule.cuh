@@ -686,22 +686,20 @@ struct Mol32 {
       box_muller(w.w[0], w.w[1], n0, n1);
       box_muller(w.w[2], w.w[3], n2, n3);
       box_muller(w.w[4], w.w[5], n4, n5);
-      const double* vp = R.vd.p;
-      vx = __fmaf_rn(float(vp[1]), n0, float(vp[0]));
-      vy = __fmaf_rn(float(vp[3]), n1, float(vp[2]));
-      vz = __fmaf_rn(float(vp[5]), n2, float(vp[4]));
-      const double* xp = R.xd.p;
+      vx = __fmaf_rn(R.vf[1], n0, R.vf[0]);
+      vy = __fmaf_rn(R.vf[3], n1, R.vf[2]);
+      vz = __fmaf_rn(R.vf[5], n2, R.vf[4]);
       if (R.xd.kind == CTRAJ_DIST_DISC_POSITION) {
         float s, c;
         sincospif(2.0f * u01f(w.w[6]), &s, &c);
-        const float rr = __fmul_rn(sqrtf(u01f(w.w[7])), float(xp[0] * 0.5));
+        const float rr = __fmul_rn(sqrtf(u01f(w.w[7])), R.xf[0]);
         x = __fmul_rn(rr, c);
         y = __fmul_rn(rr, s);
-        z_ic = xp[1];
+        z_ic = R.xd.p[1];
       } else {
-        x = __fmul_rn(float(xp[0]), n3);
-        y = __fmul_rn(float(xp[1]), n4);
-        z_ic = xp[2];
+        x = __fmul_rn(R.xf[0], n3);
+        y = __fmul_rn(R.xf[1], n4);
+        z_ic = R.xd.p[2];
       }
       gap0 = R.gap0f;
     } else {
@@ -732,17 +730,16 @@ struct Mol32 {
     float n0, n1, n2, n3;
     box_muller(a.v[0], a.v[1], n0, n1);
     box_muller(a.v[2], a.v[3], n2, n3);
-    const double* vp = R.vd.p;
-    vx = __fmaf_rn(float(vp[1]), n0, float(vp[0]));
-    vy = __fmaf_rn(float(vp[3]), n1, float(vp[2]));
-    vz = __fmaf_rn(float(vp[5]), n2, float(vp[4]));
-    x = __fmul_rn(float(R.xd.p[0]), n3);
+    vx = __fmaf_rn(R.vf[1], n0, R.vf[0]);
+    vy = __fmaf_rn(R.vf[3], n1, R.vf[2]);
+    vz = __fmaf_rn(R.vf[5], n2, R.vf[4]);
+    x = __fmul_rn(R.xf[0], n3);
   }
   __device__ void screen_rest(const Plan& P, const RunDev& R, int64_t i) {
     const Philox4 b = philox4x32_10(R.offset + uint64_t(i), 1u, R.key);
     float n4, n5;
     box_muller(b.v[0], b.v[1], n4, n5);
-    y = __fmul_rn(float(R.xd.p[1]), n4);
+    y = __fmul_rn(R.xf[1], n4);
     id = int32_t(i);
     margin = INFINITY;
     rows = 0;

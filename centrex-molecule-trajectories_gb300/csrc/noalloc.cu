@@ -338,6 +338,7 @@ extern "C" int ctraj_run_noalloc(const ctraj_element* el, int32_t n_el, int32_t 
   R.ic_mode = a->ic_mode;
   R.xd = a->xdist;
   R.vd = a->vdist;
+  round_distributions(R);
   R.ics = a->ics;
   if (a->ic_mode == CTRAJ_IC_DEVICE_DRAW) {
     const double zd = a->xdist.kind == CTRAJ_DIST_DISC_POSITION ? a->xdist.p[1] : a->xdist.p[2];

@@ -118,7 +118,8 @@ struct RunDev {
   const double* ics;  // (6, n) when injected
   ctraj_distribution xd, vd;
   float gap0f;         // FP32 first flight for drawn ICs: (float)(el[0].z0 - xd.z)
-  float pad3;
+  float xf[3], vf[6];  // xd.p (a disc: radius and z) and vd.p rounded to float: a conversion in the
+                       // kernel takes the FP64 pipe, per molecule where it is not hoisted
   int32_t* out_label;
   double* out_final;   // (10, n)
   int32_t* out_rows;
@@ -210,6 +211,15 @@ constexpr int kCtlWords = 4;
 struct SweepQueues {
   Queue q[CTRAJ_MAX_TABLES];
 };
+
+// R.xf and R.vf from the distributions.
+inline void round_distributions(RunDev& R) {
+  const bool disc = R.xd.kind == CTRAJ_DIST_DISC_POSITION;
+  R.xf[0] = float(disc ? R.xd.p[0] * 0.5 : R.xd.p[0]);
+  R.xf[1] = float(R.xd.p[1]);
+  R.xf[2] = float(R.xd.p[2]);
+  for (int k = 0; k < 6; ++k) R.vf[k] = float(R.vd.p[k]);
+}
 
 constexpr int kLabelDetected = -1;  // counts[n_labels]
 constexpr int kQueued = -2;         // waiting at a lens entrance
