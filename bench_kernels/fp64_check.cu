@@ -1,6 +1,7 @@
 // Part of libctraj_probes.so (bench_kernels/).  Checks of the square roots and
 // quotients the kernels form themselves.  The lens pass's FP32 root (sqrt32)
-// against sqrtf for every float of its range; the exact mode's FP64
+// against sqrtf for every float of its range; the soft lens pass's edge test
+// (soft_test_r2) against the general one; the exact mode's FP64
 // forms (fp64.cuh) against the IEEE operations they stand for, over generated
 // operands: random significands with exponents of the lens pass and of the
 // whole allowed range, significands near all-zeros and all-ones, and operands
@@ -8,6 +9,7 @@
 // and their neighbours).
 #include <cuda_runtime.h>
 
+#include "adjoint.cuh"
 #include "fp64.cuh"
 #include "molecule.cuh"
 
@@ -84,7 +86,32 @@ __global__ void k_sqrt32_check(unsigned long long* bad) {
   if (b) atomicAdd(bad, b);
 }
 
+// every y >= 0, infinity and a NaN, x = 0, at an edge of radius R and width 1 / inv_w
+__global__ void k_soft_test_check(float R, float inv_w, unsigned long long* bad) {
+  unsigned long long b = 0;
+  auto same = [](float p, float q) { return p == q || (isnan(p) && isnan(q)); };
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k <= 0x7f800001u; k += gridDim.x * blockDim.x) {
+    const float y = __uint_as_float(k);
+    float ls, d, ls2, d2;
+    ctraj::soft_test(0.0f, y, R, inv_w, ls, d);
+    ctraj::soft_test_r2(__fmaf_rn(y, y, 0.0f), R, inv_w, ls2, d2);
+    b += same(ls, ls2) && same(d, d2) ? 0 : 1;
+  }
+  if (b) atomicAdd(bad, b);
+}
+
 }  // namespace
+
+extern "C" int ctraj_peak_soft_test_check(float R, float inv_w, unsigned long long* mismatches) {
+  if (!mismatches) return -1;
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, sizeof *d) != cudaSuccess) return -3;
+  cudaMemset(d, 0, sizeof *d);
+  k_soft_test_check<<<1216, 256>>>(R, inv_w, d);
+  cudaError_t e = cudaMemcpy(mismatches, d, sizeof *d, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : -2;
+}
 
 extern "C" int ctraj_peak_sqrt32_check(unsigned long long* mismatches) {
   if (!mismatches) return -1;

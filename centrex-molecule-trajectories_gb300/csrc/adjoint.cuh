@@ -140,6 +140,30 @@ __device__ __forceinline__ void soft_test(T x, T y, T R, T inv_w, T& ls, T& d) {
   d = mul_(dls, inv_w);
 }
 
+// soft_test of a state given by its squared radius.  FP32: the same values
+// without the care of the general rsqrt and division for subnormal and huge
+// operands, which here are neither but for r2 < 2^-126 (r is taken as 0), and
+// with log sigma(z) = min(z, 0) - log(1 + e).
+__device__ __forceinline__ void soft_test_r2(float r2, float R, float inv_w, float& ls, float& d) {
+  auto rcp = [](float v) {
+    float h;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(h) : "f"(v));
+    return h;
+  };
+  float h;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(h) : "f"(r2));
+  const float r = r2 >= 0x1p-126f ? mul_(r2, h) : 0.0f;  // 0 for a NaN too, as soft_radius
+  const float z = mul_(add_(R, -r), inv_w), e = exp_(-fabsf(z));
+  const float s = mul_(e, rcp(add_(2.0f, e)));
+  ls = add_(fminf(z, 0.0f), -log1p_series(s));
+  d = mul_(mul_(z >= 0.0f ? e : 1.0f, rcp(add_(1.0f, e))), inv_w);
+}
+__device__ __forceinline__ void soft_test_r2(double r2, double R, double inv_w, double& ls, double& d) {
+  double dls;
+  log_sigmoid(mul_(add_(R, -sqrt_(r2)), inv_w), ls, dls);
+  d = mul_(dls, inv_w);
+}
+
 // Launch-time constants of a soft run.
 struct SoftPlan {
   int64_t n;                        // molecules of the whole run
@@ -701,11 +725,15 @@ __device__ __forceinline__ void stage_table(const SoftPlan& S, const Coef4<T>* t
 // and the queue of molecules that stay above the floor.  The floor test runs
 // every 8 steps (the log weight only decreases, so the dropped set is the
 // same) to keep it off the step-to-step dependency chain.
+// The four CTAs per SM in the launch bounds are for the compiler's choice of
+// registers: with 118 to 125 it interleaves the groups below, left to itself it
+// may settle on 96, and a group then takes half as long again (loss of 1e6
+// molecules in a focusing lens: 773 instead of 1000 us in the lens pass).
 template <class T, bool kGrad>
-__global__ void __launch_bounds__(kSoftThreads) k_soft_lens(const __grid_constant__ SoftPlan S, const SoftQueue Q,
-                                                            const Coef4<T>* __restrict__ table, T* ckpt,
-                                                            size_t cap, double* __restrict__ contrib,
-                                                            unsigned long long* stats) {
+__global__ void __launch_bounds__(kSoftThreads, 4) k_soft_lens(const __grid_constant__ SoftPlan S, const SoftQueue Q,
+                                                               const Coef4<T>* __restrict__ table, T* ckpt,
+                                                               size_t cap, double* __restrict__ contrib,
+                                                               unsigned long long* stats) {
   extern __shared__ unsigned char s_raw[];
   Coef4<T>* s_tab = reinterpret_cast<Coef4<T>*>(s_raw);
   stage_table(S, table, s_tab);
@@ -745,30 +773,38 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens(const __grid_constan
       // steps run beside the bore tests of the previous group's 8 states,
       // which do not depend on them, so the two chains' latencies overlap
       // (with the branch-free FP32 log sigmoid, the slowest molecule's step
-      // 550 -> ~370 cycles); the tests are added to the log
+      // 550 -> ~250 cycles); the tests are added to the log
       // weight in step order, as one at a time would add them.  The floor
       // test after a group sees the tests up to the previous group: the log
       // weight only decreases, so the same molecules are dropped, up to 8
       // steps later.  Checkpoints between groups.
-      T qx[8], qy[8];
+      T q[8];  // squared radii of the states before steps pn .. pn + 7
 #pragma unroll
-      for (int u = 0; u < 8; ++u) qx[u] = qy[u] = T(0);
-      bool pend = false;  // qx, qy hold the states before steps pn .. pn + 7
+      for (int u = 0; u < 8; ++u) q[u] = T(0);
+      bool pend = false;  // there are some
       int pn = 0;
+      auto test = [&](int u) {
+        T ls, d;
+        soft_test_r2(q[u], bore, inv_w, ls, d);
+        if (u == 0) {  // not the entrance, which m.front tested
+          ls = pn > 0 ? ls : T(0);
+          d = pn > 0 ? d : T(0);
+        }
+        m.lw = add_(m.lw, ls);
+        m.d_bore = add_(m.d_bore, d);
+      };
       for (; n + 8 <= L.N; n += 8) {
         if (kGrad && n % K == 0) store_ckpt(n);
+        const T lw = m.lw, d_bore = m.d_bore;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const T sx = x, sy = y;
+          const T r2 = fma_(y, y, mul_(x, x));
           soft_step<T, true>(C, s_tab, x, y, vx, vy, cx, cy, cvx, cvy, L.dt, L.hdt, L.c2, L.dt6, L.dt26, nullptr);
-          T ls, d;
-          soft_test(qx[u], qy[u], bore, inv_w, ls, d);
-          const bool use = pend && pn + u > 0;
-          m.lw = add_(m.lw, use ? ls : T(0));
-          m.d_bore = add_(m.d_bore, use ? d : T(0));
-          qx[u] = sx;
-          qy[u] = sy;
+          test(u);
+          q[u] = r2;
         }
+        m.lw = pend ? m.lw : lw;
+        m.d_bore = pend ? m.d_bore : d_bore;
         pend = true;
         pn = n;
         if (!(m.lw >= floor_)) {
@@ -779,12 +815,7 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens(const __grid_constan
       }
       if (alive && pend) {  // the last group's tests
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          T ls, d;
-          soft_test(qx[u], qy[u], bore, inv_w, ls, d);
-          m.lw = add_(m.lw, pn + u > 0 ? ls : T(0));
-          m.d_bore = add_(m.d_bore, pn + u > 0 ? d : T(0));
-        }
+        for (int u = 0; u < 8; ++u) test(u);
         if (!(m.lw >= floor_)) alive = false;
       }
     }
@@ -1071,10 +1102,10 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_seg(const __grid_constant
 // (recomputed): d lw / d(lens z0) from the last flight time, d lw / d(sigma_v)
 // from the initial velocities.  Adds the weighted terms to contrib.
 template <class T>
-__global__ void __launch_bounds__(kSoftThreads) k_soft_compose(const __grid_constant__ SoftPlan S, const SoftQueue Q,
-                                                               const T* __restrict__ seg_out, int max_seg,
-                                                               double* __restrict__ contrib,
-                                                               size_t cap) {
+__global__ void __launch_bounds__(kSoftThreads, 1) k_soft_compose(const __grid_constant__ SoftPlan S, const SoftQueue Q,
+                                                                  const T* __restrict__ seg_out, int max_seg,
+                                                                  double* __restrict__ contrib,
+                                                                  size_t cap) {
   const unsigned nb = *Q.bcount;
   const T inv_w = T(S.inv_w), bore = T(S.bore);
   for (unsigned b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
@@ -1094,7 +1125,9 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_compose(const __grid_cons
     }
     // unrolled so that the next segments' loads are issued while this one's
     // products wait (a thread walks its segments in order; the maps are read
-    // once each): 1e6 drawn molecules 66 us by twos, 48 by fours
+    // once each), and with the registers to hold them (the launch bounds; the
+    // compiler by itself settled on 62 in FP32): 1e6 drawn molecules 66 us by
+    // twos, 27 by fours
 #pragma unroll 4
     for (int sg = n_seg - 1; sg >= 0; --sg) {
       T o[kSoftSegStride];

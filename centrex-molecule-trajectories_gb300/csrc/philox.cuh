@@ -68,8 +68,7 @@ __host__ __device__ inline Philox4 philox4x32_10(uint64_t ctr, uint32_t call, co
 // log(1 + x) for x in [-1/2, 1], branch-free: 2 atanh(s) with s = x / (2 + x)
 // in [-1/3, 1/3], from the series 2 s (1 + s^2/3 + s^4/5 + ... + s^14/15),
 // whose next term is below 1.4e-9 relative; s by the fast division (2 ulp).
-__device__ __forceinline__ float log1p_atanh(float x) {
-  const float s = __fdividef(x, __fadd_rn(2.0f, x));
+__device__ __forceinline__ float log1p_series(float s) {
   const float s2 = __fmul_rn(s, s);
   float p = 1.0f / 15.0f;
   p = __fmaf_rn(p, s2, 1.0f / 13.0f);
@@ -81,6 +80,7 @@ __device__ __forceinline__ float log1p_atanh(float x) {
   p = __fmaf_rn(p, s2, 1.0f);
   return __fmul_rn(__fmul_rn(2.0f, s), p);
 }
+__device__ __forceinline__ float log1p_atanh(float x) { return log1p_series(__fdividef(x, __fadd_rn(2.0f, x))); }
 
 // sin(pi a) and cos(pi a) for a in [0, 2], branch-free: a = j/2 + f with
 // j = rint(2a) and |f| <= 1/4 (f exact), x = pi f, the Taylor series of sin

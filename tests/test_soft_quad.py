@@ -2,7 +2,10 @@
 (k_soft_lens_quad) and one beyond: a run whose queue is long must equal the sum
 of its parts whose queues are short, counts exactly, loss and gradient to the
 rounding of their sums; without whole eights between checkpoints every queue
-takes the one-lane pass."""
+takes the one-lane pass.  The FP32 pass's edge test (soft_test_r2) must give
+the general one's values."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -42,3 +45,16 @@ def test_long_queue_equals_its_parts(low, detector, dt_scale):
         assert np.abs(a.grad - c.grad).max() <= 1e-10 * np.abs(c.grad).max()
     finally:
         eng.close()
+
+
+# widths from a ten-thousandth of the radius to a hundred times it, and an edge of radius 0: every float radius, of which
+# the smallest have a square below the normal numbers
+@pytest.mark.parametrize("radius,inv_w", [(0.0222, 5e3), (0.0175, 1.0), (1e-3, 1e7), (1.0, 1e2), (0.0, 1.0)])
+def test_the_lens_pass_edge_test_is_the_general_one(radius, inv_w):
+    from bench_kernels.build import build as build_probes
+
+    lib = ctypes.CDLL(str(build_probes()))
+    lib.ctraj_peak_soft_test_check.argtypes = [ctypes.c_float, ctypes.c_float, ctypes.POINTER(ctypes.c_ulonglong)]
+    bad = ctypes.c_ulonglong(1)
+    assert lib.ctraj_peak_soft_test_check(radius, inv_w, ctypes.byref(bad)) == 0
+    assert bad.value == 0
