@@ -91,6 +91,38 @@ __global__ void k_bm_check(const long long n, float* out) {
 }  // namespace
 
 // Returns 0 and the six largest errors above (out[6]) over n arguments.
+// out[0]: words w for which box_muller_pair differs from two box_muller calls
+// (w as U1 and as U2, in both components)
+namespace {
+__global__ void k_bm_pair_check(unsigned long long* bad) {
+  unsigned long long b = 0;
+  for (unsigned long long k = blockIdx.x * blockDim.x + threadIdx.x; k < (1ull << 32); k += gridDim.x * blockDim.x) {
+    const unsigned w = unsigned(k), v = mix(w);
+    float2 p, q;
+    ctraj::box_muller_pair(make_uint2(w, v), make_uint2(v, w), p, q);
+    float a, c, d, e;
+    ctraj::box_muller(w, v, a, c);
+    ctraj::box_muller(v, w, d, e);
+    b += __float_as_uint(a) == __float_as_uint(p.x) && __float_as_uint(c) == __float_as_uint(q.x) &&
+                 __float_as_uint(d) == __float_as_uint(p.y) && __float_as_uint(e) == __float_as_uint(q.y)
+             ? 0
+             : 1;
+  }
+  if (b) atomicAdd(bad, b);
+}
+}  // namespace
+
+extern "C" int ctraj_peak_bm_pair_check(unsigned long long* mismatches) {
+  if (!mismatches) return -1;
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, sizeof *d) != cudaSuccess) return -3;
+  cudaMemset(d, 0, sizeof *d);
+  k_bm_pair_check<<<1216, 256>>>(d);
+  cudaError_t e = cudaMemcpy(mismatches, d, sizeof *d, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : -2;
+}
+
 extern "C" int ctraj_peak_bm_check(long long n, float* out) {
   if (n < 1 || !out) return -1;
   float* d = nullptr;

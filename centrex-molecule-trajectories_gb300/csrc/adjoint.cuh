@@ -309,9 +309,13 @@ struct SoftMol {
     if (S.ic_mode == CTRAJ_IC_DEVICE_DRAW) {
       const Words8 w = molecule_words(S.offset + uint64_t(i), S.key);
       T n5;
-      box_muller(w.w[0], w.w[1], n0, n1);
-      box_muller(w.w[2], w.w[3], n2, n3);
+      typename std::conditional<std::is_same<T, float>::value, float2, double2>::type n02, n13;
+      box_muller_pair(make_uint2(w.w[0], w.w[2]), make_uint2(w.w[1], w.w[3]), n02, n13);
       box_muller(w.w[4], w.w[5], n4, n5);
+      n0 = n02.x;
+      n1 = n13.x;
+      n2 = n02.y;
+      n3 = n13.y;
     } else {
       const size_t n = size_t(S.n), k = size_t(i);
       n0 = T(S.normals[k]);

@@ -233,8 +233,8 @@ __device__ __forceinline__ void ring_entry(const ctraj_ring& G, unsigned long lo
 // Screening (FP32 runs without per-molecule outputs, device draws with a
 // Gaussian position, element 0 a circular or rectangular aperture): most
 // molecules of such a beamline are stopped at element 0's entrance plane by
-// their x alone, which the first of a molecule's two Philox calls decides
-// (Mol32::screened_out).  Those are tallied there; the others wait in a
+// their x and vy, which the first of a molecule's two Philox calls decides
+// whatever their y within its bound (Mol32::screened_out).  Those are tallied there; the others wait in a
 // per-warp buffer (index, vx, vy, vz, x) and are taken 32 at a time, in full
 // warps, for the second call and the walk -- the same results as the full
 // walk of every molecule, with the second call, a Box-Muller pair and the
@@ -348,6 +348,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_front(const __grid_constan
   }
   if (screen) {
     if constexpr (M::kScreenable) {
+      const typename M::Screen sc = M::screen(P, R);
       int waiting = 0;  // warp-uniform: molecules in this warp's buffer
       unsigned screened = 0;  // and those stopped by the screening
       // the last k waiting molecules, one per lane, through the walk
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_front(const __grid_constan
         bool wait = false;
         if (i < R.n) {
           m.screen_draw(R, i);
-          wait = !m.screened_out(P, R.gap0f);
+          wait = !m.screened_out(P, R.gap0f, sc);
         }
         const unsigned wm = __ballot_sync(kFull, wait);
         if (wait) scr[waiting + __popc(wm & lanes_lt)] = ScreenSlot{int32_t(i), m.vx, m.vy, m.vz, m.x};
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_sweep_front(const __grid_c
   }
   if (screen) {
     if constexpr (M::kScreenable) {
+      const typename M::Screen sc = M::screen(P, R);
       int waiting = 0;  // warp-uniform
       auto take = [&](const int k) {  // the last k waiting molecules, one per lane
         M m;
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(kFrontMaxThreads) k_sweep_front(const __grid_c
         bool wait = false, out = false;
         if (i < hi) {
           m.screen_draw(R, i);
-          out = m.screened_out(P, R.gap0f);
+          out = m.screened_out(P, R.gap0f, sc);
           wait = !out;
         }
         // the 32 molecules' configurations, one after the other
