@@ -253,7 +253,7 @@ PersistKernel persist_kernel(bool out, int force, int mode, bool staged, int lan
 template <int F>  // one force law's configurations (k_persist_<law>.cu)
 PersistKernel persist_kernel_for(bool out, int mode, bool staged, int lanes, int mpt, int* threads, int* used_mpt);
 
-// k_lens_finish for a plain, batch or sweep pass (k_persist.cu).
+// k_lens_finish for a plain or batch pass (k_persist.cu).
 using FinishKernel = void (*)(const Plan, const RunDev, const int, const Queue, const Queue, const DoneRec*,
                               const unsigned);
 FinishKernel finish_kernel(int mode);

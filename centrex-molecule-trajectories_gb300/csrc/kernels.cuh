@@ -782,8 +782,8 @@ __device__ __forceinline__ void order_range(unsigned n, unsigned& lo, unsigned& 
   hi = min(n, lo + per);
 }
 
-static __global__ void __launch_bounds__(kOrderThreads) k_order_count(const __grid_constant__ Plan P, const int li,
-                                                               const Queue Q, unsigned* hist, const int outward) {
+__device__ __forceinline__ void order_count(const Plan& P, const int li, const Queue& Q, unsigned* hist,
+                                            const int outward) {
   __shared__ unsigned h[kOrderBuckets];
   for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x) h[b] = 0;
   __syncthreads();
@@ -796,8 +796,14 @@ static __global__ void __launch_bounds__(kOrderThreads) k_order_count(const __gr
   for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x)
     if (h[b]) atomicAdd(hist + b, h[b]);
 }
+static __global__ void __launch_bounds__(kOrderThreads) k_order_count(const __grid_constant__ Plan P, const int li,
+                                                               const Queue Q, unsigned* hist, const int outward) {
+  order_count(P, li, Q, hist, outward);
+}
 
-static __global__ void __launch_bounds__(kOrderBuckets) k_order_scan(unsigned* hist) {
+// Block b scans the buckets of queue b (a sweep has one per Stark table).
+static __global__ void __launch_bounds__(kOrderBuckets) k_order_scan(unsigned* hists) {
+  unsigned* hist = hists + size_t(blockIdx.x) * kOrderBuckets;
   __shared__ unsigned t[kOrderBuckets];
   const int i = threadIdx.x;
   const unsigned own = hist[i];
@@ -815,9 +821,8 @@ static __global__ void __launch_bounds__(kOrderBuckets) k_order_scan(unsigned* h
 // Same ranges as k_order_count: the block reserves its entries of every
 // bucket with one global atomic per bucket, then places them with
 // shared-memory atomics.
-static __global__ void __launch_bounds__(kOrderThreads) k_order_place(const __grid_constant__ Plan P, const int li,
-                                                               const Queue Q, unsigned* cursor, unsigned* order,
-                                                               const int outward) {
+__device__ __forceinline__ void order_place(const Plan& P, const int li, const Queue& Q, unsigned* cursor,
+                                            unsigned* order, const int outward) {
   __shared__ unsigned h[kOrderBuckets];
   for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x) h[b] = 0;
   __syncthreads();
@@ -832,6 +837,11 @@ static __global__ void __launch_bounds__(kOrderThreads) k_order_place(const __gr
   __syncthreads();
   for (unsigned j = lo + threadIdx.x; j < hi; j += blockDim.x)
     order[atomicAdd(h + order_bucket(P.el[li], Q, j, scale, outward), 1u)] = j;
+}
+static __global__ void __launch_bounds__(kOrderThreads) k_order_place(const __grid_constant__ Plan P, const int li,
+                                                               const Queue Q, unsigned* cursor, unsigned* order,
+                                                               const int outward) {
+  order_place(P, li, Q, cursor, order, outward);
 }
 
 // ---------------------------------------------------------------------------
@@ -1453,9 +1463,8 @@ __global__ void __launch_bounds__(kT, 1) k_lens_persist(const __grid_constant__ 
 constexpr int kFinishThreads = 256;
 
 template <class M, int kMode>
-__global__ void __launch_bounds__(kFinishThreads) k_lens_finish(const __grid_constant__ Plan P, const RunDev R,
-                                                                const int li, const Queue Qin, const Queue Qnext,
-                                                                const DoneRec* done, const unsigned cap) {
+__device__ __forceinline__ void lens_finish_queue(const Plan& P, const RunDev& R, const int li, const Queue& Qin,
+                                                  const Queue& Qnext, const DoneRec* done, const unsigned cap) {
   __shared__ BlockTally S;
   tally_init(S);
   __syncthreads();
@@ -1497,6 +1506,12 @@ __global__ void __launch_bounds__(kFinishThreads) k_lens_finish(const __grid_con
   }
   if (kMode != kModeBatch) persist_flush(S, R, P.n_labels, acc);
 }
+template <class M, int kMode>
+__global__ void __launch_bounds__(kFinishThreads) k_lens_finish(const __grid_constant__ Plan P, const RunDev R,
+                                                                const int li, const Queue Qin, const Queue Qnext,
+                                                                const DoneRec* done, const unsigned cap) {
+  lens_finish_queue<M, kMode>(P, R, li, Qin, Qnext, done, cap);
+}
 
 // Batched sweep: the Stark tables' lens queues in one launch.  Each CTA
 // starts on a table, chosen so that CTAs are spread over the tables in
@@ -1505,12 +1520,35 @@ __global__ void __launch_bounds__(kFinishThreads) k_lens_finish(const __grid_con
 // (one CTA per SM).
 struct SweepTabs {
   const float4* q[CTRAJ_MAX_TABLES];
-  const unsigned* order[CTRAJ_MAX_TABLES];
+  unsigned* order[CTRAJ_MAX_TABLES];
   float s0[CTRAJ_MAX_TABLES];
   int n_int[CTRAJ_MAX_TABLES];
   DoneRec* done[CTRAJ_MAX_TABLES];         // deferred molecule ends (nullptr: none)
   unsigned done_cap[CTRAJ_MAX_TABLES];     // queue positions with a record
 };
+
+// The entrants' order and the deferred ends of a sweep: k_order_count, k_order_place and k_lens_finish for all tables in
+// one launch each, table blockIdx.y.  Launches of a few microseconds on a part of the chip otherwise, four per table:
+// 256 configurations of four tables, 142 -> 68 us.  Buckets of table t: hists + t kOrderBuckets.
+static __global__ void __launch_bounds__(kOrderThreads) k_sweep_order_count(const __grid_constant__ Plan P, const int li,
+                                                                     const __grid_constant__ SweepQueues Qs,
+                                                                     unsigned* hists, const int outward) {
+  order_count(P, li, Qs.q[blockIdx.y], hists + size_t(blockIdx.y) * kOrderBuckets, outward);
+}
+static __global__ void __launch_bounds__(kOrderThreads) k_sweep_order_place(const __grid_constant__ Plan P, const int li,
+                                                                     const __grid_constant__ SweepQueues Qs,
+                                                                     unsigned* cursors,
+                                                                     const __grid_constant__ SweepTabs T,
+                                                                     const int outward) {
+  const int t = blockIdx.y;
+  order_place(P, li, Qs.q[t], cursors + size_t(t) * kOrderBuckets, T.order[t], outward);
+}
+static __global__ void __launch_bounds__(kFinishThreads) k_sweep_finish(const __grid_constant__ Plan P, const RunDev R,
+                                                                 const int li, const __grid_constant__ SweepQueues Qs,
+                                                                 const __grid_constant__ SweepTabs T) {
+  const int t = blockIdx.y;
+  lens_finish_queue<Mol32<false, false>, kModeSweep>(P, R, li, Qs.q[t], Qs.q[t], T.done[t], T.done_cap[t]);
+}
 
 template <int F, bool kStaged, int kT = kPersistThreads>
 __global__ void __launch_bounds__(kT, 1) k_sweep_persist(const __grid_constant__ Plan P, const RunDev R,
@@ -1528,10 +1566,11 @@ __global__ void __launch_bounds__(kT, 1) k_sweep_persist(const __grid_constant__
   int max_int = 0;
   for (int t = 0; t < n_tab; ++t) max_int = max(max_int, T.n_int[t]);
   SwapSlot* s_swap = reinterpret_cast<SwapSlot*>(s_dyn + (kStaged ? max_int : 0));
-  tally_init(S);
   // first table: the one whose share of the queued molecules holds this CTA's
   unsigned total = 0;
   for (int t = 0; t < n_tab; ++t) total += *(volatile unsigned*)Qs.q[t].count;
+  if (total < L0.min_count || total > L0.max_count) return;
+  tally_init(S);
   const float pos = (float(blockIdx.x) + 0.5f) / float(gridDim.x) * float(total);
   int t0 = n_tab - 1;
   for (unsigned cum = 0, t = 0; t < unsigned(n_tab); ++t) {

@@ -59,7 +59,7 @@ struct LensArgs {
   float bore;   // d/2
   int classic;
   int outward;  // LensF::outward
-  unsigned min_count, max_count;  // k_lens_persist: queue sizes this launch takes
+  unsigned min_count, max_count;  // k_lens_persist, k_sweep_persist: queued molecules this launch takes
 };
 
 // FP64 view of a force table (device pointers).

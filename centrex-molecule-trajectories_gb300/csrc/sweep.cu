@@ -80,7 +80,8 @@ struct SweepLaunch {
   bool persistent = false;               // one k_sweep_persist launch instead of the chunks
   int force = kForceStark2;              // the lens's force law; kForceStark2Lin when every table
                                          // passes the linear form's test at its largest voltage
-  unsigned* order[CTRAJ_MAX_TABLES] = {};  // persistent: bucket counts then entrant order, per table
+  unsigned* hists = nullptr;               // persistent: bucket counts, kOrderBuckets per table
+  unsigned* order[CTRAJ_MAX_TABLES] = {};  // persistent: entrant order, per table
   DoneRec* done[CTRAJ_MAX_TABLES] = {};    // persistent: the molecules' end records, per table
   unsigned done_cap[CTRAJ_MAX_TABLES] = {};
   int outward = 0;                         // every configuration's force points away from the axis
@@ -110,10 +111,19 @@ bool sweep_staged(const SweepLaunch& W) {
   return true;
 }
 
-size_t sweep_persist_smem(const SweepLaunch& W) {
+// A sweep's linear pass with 512 lanes per CTA (the default) takes 768 for more queued molecules than kSweepWideRounds
+// rounds of 512: more warps per scheduler hide more of a step's latency, but a molecule's own steps take longer, which is
+// what a short queue waits for.  Rounds 3.3, 4.4, 6.7, 8.9, 22: 1.13, 1.08, 0.98, 0.97, 0.94 of the time with 512.  The
+// count is known on the device only, so both are launched and one returns.
+constexpr int kSweepWideThreads = 768, kSweepWideRounds = 6;
+bool sweep_wide(const SweepLaunch& W) {
+  return W.force == kForceStark2Lin && sweep_staged(W) && W.threads == kPersistThreads;
+}
+
+size_t sweep_persist_smem(const SweepLaunch& W, int threads) {
   int max_int = 0;
   for (int t = 0; t < W.n_tab; ++t) max_int = std::max(max_int, W.la[t].n_int);
-  return (sweep_staged(W) ? size_t(max_int) * sizeof(float4) : 0) + size_t(W.threads) * sizeof(SwapSlot);
+  return (sweep_staged(W) ? size_t(max_int) * sizeof(float4) : 0) + size_t(threads) * sizeof(SwapSlot);
 }
 
 // The whole sweep on c->stream (forking to one side stream per table).  Every
@@ -147,32 +157,40 @@ int sweep_enqueue(ctraj_context* c, const Plan& P, const RunDev& R, const SweepL
     SweepTabs T{};
     for (int t = 0; t < W.n_tab; ++t) {
       Qs.q[t] = W.qa[t];
-      unsigned* hist = W.order[t];
-      CT_CUDA(cudaMemsetAsync(hist, 0, kOrderBuckets * sizeof(unsigned), s));
-      k_order_count<<<c->sm_count, kOrderThreads, 0, s>>>(P, W.lens, W.qa[t], hist, W.outward);
-      k_order_scan<<<1, kOrderBuckets, 0, s>>>(hist);
-      k_order_place<<<c->sm_count, kOrderThreads, 0, s>>>(P, W.lens, W.qa[t], hist, hist + kOrderBuckets,
-                                                          W.outward);
-      CT_CUDA(cudaGetLastError());
-      launches += 3;
       T.q[t] = W.la[t].q;
-      T.order[t] = hist + kOrderBuckets;
+      T.order[t] = W.order[t];
       T.s0[t] = W.la[t].s0;
       T.n_int[t] = W.la[t].n_int;
       T.done[t] = W.done[t];
       T.done_cap[t] = W.done_cap[t];
     }
-    sweep_persist_kernel(W.force, sweep_staged(W), W.threads)<<<c->sm_count, W.threads,
-                                                                             sweep_persist_smem(W), s>>>(
-        P, R, W.lens, Qs, W.n_tab, T, W.la[0], c->lens_interval, c->lens_service);
+    CT_CUDA(cudaMemsetAsync(W.hists, 0, size_t(W.n_tab) * kOrderBuckets * sizeof(unsigned), s));
+    const dim3 grid(unsigned(c->sm_count), unsigned(W.n_tab));
+    k_sweep_order_count<<<grid, kOrderThreads, 0, s>>>(P, W.lens, Qs, W.hists, W.outward);
+    k_order_scan<<<W.n_tab, kOrderBuckets, 0, s>>>(W.hists);
+    k_sweep_order_place<<<grid, kOrderThreads, 0, s>>>(P, W.lens, Qs, W.hists, T, W.outward);
+    CT_CUDA(cudaGetLastError());
+    launches += 3;
+    auto pass = [&](int threads, unsigned min_count, unsigned max_count) {
+      LensArgs L = W.la[0];
+      L.min_count = min_count;
+      L.max_count = max_count;
+      sweep_persist_kernel(W.force, sweep_staged(W), threads)<<<c->sm_count, threads, sweep_persist_smem(W, threads), s>>>(
+          P, R, W.lens, Qs, W.n_tab, T, L, c->lens_interval, c->lens_service);
+      ++launches;
+      return cudaGetLastError();
+    };
+    if (sweep_wide(W)) {
+      const unsigned few = unsigned(c->sm_count) * kPersistThreads * kSweepWideRounds;
+      CT_CUDA(pass(W.threads, 0u, few));
+      CT_CUDA(pass(kSweepWideThreads, few + 1u, 0xFFFFFFFFu));
+    } else {
+      CT_CUDA(pass(W.threads, 0u, 0xFFFFFFFFu));
+    }
+    // the molecules' ends, in full warps
+    k_sweep_finish<<<dim3(unsigned(c->sm_count) * 8u, unsigned(W.n_tab)), kFinishThreads, 0, s>>>(P, R, W.lens, Qs, T);
     CT_CUDA(cudaGetLastError());
     ++launches;
-    for (int t = 0; t < W.n_tab; ++t) {  // the molecules' ends, in full warps
-      finish_kernel(kModeSweep)<<<c->sm_count * 8, kFinishThreads, 0, s>>>(P, R, W.lens, Qs.q[t], Qs.q[t],
-                                                                          W.done[t], W.done_cap[t]);
-      CT_CUDA(cudaGetLastError());
-      ++launches;
-    }
     if (c->timing) CT_CUDA(record(c->ev[3]));
     CT_CUDA(cudaMemcpyAsync(c->sweep_host, W.result, W.result_bytes, cudaMemcpyDeviceToHost, s));
     c->sweep_launches = launches;
@@ -339,10 +357,11 @@ extern "C" int ctraj_run_sweep(ctraj_context* c, const ctraj_sweep* sw, const ct
     size_t words_o = 0;
     for (int t = 0; t < W.n_tab; ++t) words_o += kOrderBuckets + size_t(std::max<int64_t>(tab_n[t], 1));
     if ((st = ens(c->sweep_order, words_o * sizeof(unsigned)))) return st;
-    size_t off = 0;
+    W.hists = c->sweep_order.as<unsigned>();
+    size_t off = size_t(W.n_tab) * kOrderBuckets;
     for (int t = 0; t < W.n_tab; ++t) {
-      W.order[t] = c->sweep_order.as<unsigned>() + off;
-      off += kOrderBuckets + size_t(std::max<int64_t>(tab_n[t], 1));
+      W.order[t] = W.hists + off;
+      off += size_t(std::max<int64_t>(tab_n[t], 1));
     }
     // end records for the first eighth of each table's queue (at least 2^20
     // positions): the lens entrants are a few percent of the molecules; the
@@ -492,8 +511,9 @@ extern "C" int ctraj_run_sweep(ctraj_context* c, const ctraj_sweep* sw, const ct
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   }
   if (W.persistent)
-    CT_CUDA(cudaFuncSetAttribute(sweep_persist_kernel(W.force, sweep_staged(W), W.threads),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_persist_smem(W))));
+    for (const int threads : {W.threads, sweep_wide(W) ? kSweepWideThreads : W.threads})
+      CT_CUDA(cudaFuncSetAttribute(sweep_persist_kernel(W.force, sweep_staged(W), threads),
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_persist_smem(W, threads))));
   CT_CUDA(cudaFuncSetAttribute(k_sweep_front<Mol32<false, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(sweep_front_smem(kFrontMaxThreads))));
   c->timing = timing;
