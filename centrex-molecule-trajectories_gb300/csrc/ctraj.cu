@@ -293,9 +293,11 @@ int check_beamline(const ctraj_context* c) {
   return CTRAJ_OK;
 }
 
+constexpr unsigned kWideRounds = 8, kWidestRounds = 32, kWideShare = 32;
+
 int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i, const Queue& Qin,
                        const Queue& Qnext, unsigned* order_buf, int sms, int interval, int service, cudaStream_t s,
-                       int* launches, int lanes, int mpt, DoneRec* done) {
+                       int* launches, int lanes, int mpt, DoneRec* done, unsigned by_count) {
   const bool staged = P.lf[i].n_smem > 0;
   unsigned* hist = order_buf;
   unsigned* order = hist + kOrderBuckets;
@@ -320,14 +322,28 @@ int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i
     *launches += 1;
     return CTRAJ_OK;
   };
-  // a queue that 512 lanes per CTA hold at once gains nothing from more of them,
-  // and steps faster with the registers of 512 threads: 8 runs of 3e5 molecules
-  // in groups of 4 (20 000 entrants) 1.41 ms at 1024 lanes, 1.19 at 512
-  const unsigned fits = unsigned(sms) * unsigned(kPersistThreads);
+  // Rounds of 512 lanes per CTA that the queue fills.  More lanes hide more of
+  // a step's latency; with 512 a molecule's own steps are faster, which is what
+  // a short queue waits for.  Linear form: 768 over 512 lanes at 2.8, 7, 17 and
+  // 69 rounds 1.06, 1.02, 0.92 and 0.91 of the time; 1024 over 768 1.10, 1.08,
+  // 1.03 and 0.99.  A pass without a count rule takes the lanes it is given
+  // beyond one round (8 runs of 3e5 molecules in groups of 4, 20 000 entrants:
+  // 1.41 ms at 1024 lanes, 1.19 at 512).
+  const unsigned round = unsigned(sms) * unsigned(kPersistThreads);
+  const unsigned wide = kWideRounds * round, widest = kWidestRounds * round;
   int st = CTRAJ_OK;
-  if (lanes > kPersistThreads && mpt == 1) {
-    st = pass(kPersistThreads, 1, 1u, fits);
-    if (!st) st = pass(lanes, mpt, fits + 1u, 0xFFFFFFFFu);
+  if (by_count && mpt == 1 && staged && !out && P.lf[i].force == kForceStark2Lin) {
+    // A pass that returns costs 4 us: a single run's are launched for a queue
+    // that a share of its molecules may fill, its queue being a few percent of
+    // them; a group's, whose queue is a whole group's, for one that all may.
+    const unsigned most = mode == kModeBatch ? by_count : by_count / kWideShare;
+    const bool any_wide = most > wide, any_widest = most > widest;
+    st = pass(kPersistThreads, 1, 1u, any_wide ? wide : 0xFFFFFFFFu);
+    if (!st && any_wide) st = pass(768, 1, wide + 1u, any_widest ? widest : 0xFFFFFFFFu);
+    if (!st && any_widest) st = pass(1024, 1, widest + 1u, 0xFFFFFFFFu);
+  } else if (lanes > kPersistThreads && mpt == 1) {
+    st = pass(kPersistThreads, 1, 1u, round);
+    if (!st) st = pass(lanes, mpt, round + 1u, 0xFFFFFFFFu);
   } else {
     st = pass(lanes, mpt, 1u, 0xFFFFFFFFu);
   }
@@ -420,9 +436,13 @@ int launch_persistent(ctraj_context* c, bool out, int mode, const Plan& P, const
     if ((st = c->lens_done.ensure(size_t(count) * kDoneRecBytes, 25))) return st;
     done = c->lens_done.as<DoneRec>();
   }
+  // the tuning's default lanes: by the queue's length
+  const bool batch = mode == kModeBatch;
+  const int lanes = batch ? c->batch_lens_threads : c->lens_threads;
+  const bool by_count = (batch || mode == kModePlain) && lanes == (batch ? kBatchLensThreads : kPersistThreads);
   return enqueue_persistent(out, mode, P, R, i, Qin, Qnext, c->lens_order.as<unsigned>(), c->sm_count,
-                            c->lens_interval, c->lens_service, c->stream, launches,
-                            mode == kModeBatch ? c->batch_lens_threads : c->lens_threads, c->lens_molecules, done);
+                            c->lens_interval, c->lens_service, c->stream, launches, lanes, c->lens_molecules, done,
+                            by_count ? count : 0u);
 }
 
 // k_front, then for each lens: read the lens queue's size and largest

@@ -78,6 +78,8 @@ struct HostTable {
 
 }  // namespace ctraj
 
+constexpr int kBatchLensThreads = 1024;  // default of batch_lens_threads
+
 // One context (ctraj_create): its device, stream, beamline, tables, tuning
 // and work buffers.
 struct ctraj_context {
@@ -121,7 +123,7 @@ struct ctraj_context {
   int batch_group = 4;          // ctraj_run_batch: runs sharing one lens pass
   int lens_threads = 512;       // persistent FP32 lens pass: molecule lanes per CTA
   int lens_molecules = 1;       // persistent FP32 lens pass: molecules per thread
-  int batch_lens_threads = 1024;  // lens_threads of a batch group's shared lens passes
+  int batch_lens_threads = kBatchLensThreads;  // lens_threads of a batch group's shared lens passes
   unsigned run_max_steps = 0;   // largest lens queue step bound of the last run
   bool timing = false;
   // before front, after front, before the first lens chunk, after the last one
@@ -264,9 +266,11 @@ constexpr size_t kDoneRecBytes = 64;
 // queue's entries), then one k_lens_persist launch, one CTA per SM.  With
 // `done` (kDoneRecBytes per queue entry; plain or batch passes without
 // per-molecule outputs) the molecules' ends are deferred to one k_lens_finish
-// launch after the pass.
+// launch after the pass.  by_count: the most entries Qin can hold when the
+// lanes of the linear form are to be chosen by its count (on the device: the
+// passes that it does not suit return at once), else 0.
 int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i, const Queue& Qin,
                        const Queue& Qnext, unsigned* order_buf, int sms, int interval, int service, cudaStream_t s,
-                       int* launches, int lanes, int mpt, DoneRec* done = nullptr);
+                       int* launches, int lanes, int mpt, DoneRec* done = nullptr, unsigned by_count = 0);
 
 }  // namespace ctraj
