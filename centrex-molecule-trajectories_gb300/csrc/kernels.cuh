@@ -563,7 +563,7 @@ __host__ __device__ constexpr size_t sweep_front_smem(int threads) {
 }
 
 // ---------------------------------------------------------------------------
-enum : int { kIdle = 0, kRun = 1, kLost = 2, kExit = 3, kBad = 4 };
+enum : int { kIdle = 0, kRun = 1, kLost = 2, kExit = 3, kBad = 4, kHold = 5 };
 
 // kSweep (batched sweeps, FP32 only): every molecule carries its configuration;
 // the staged table is unscaled and the configuration's beta and kappa scale it;
@@ -878,10 +878,13 @@ constexpr int kPersistService = 64;  // default steps between phase-A services
 // Steps between looks at a molecule (persist_pass).  A look costs about 170
 // cycles: the next group starts after the last step's radius and the branch on
 // it.  1e6 molecules in the focusing lens (28 per warp): 631 us with groups of
-// 4, 593 with 8, 630 with 16 (longer groups are done again more often); 1e4 (1
-// or 2 per warp): 425, 400, 382.
+// 4, 577 with 8, 797 with 16 (steps taken twice); 1e4 (1 or 2 per warp): 425,
+// 371, 362.
 constexpr int kRunGroup = 8;
 static_assert(64 % kRunGroup == 0, "groups fill 64 steps");
+// What became of a group: its steps were the molecule's, they are to be taken
+// again one at a time, or the molecule ends among them.
+enum : int { kGroupDone, kGroupAgain, kGroupEnds };
 // Phase B loads table pieces ahead while a CTA's molecules fill at most this
 // many warps: 176-212 cycles per step at one warp per scheduler against 229-264,
 // but 39.6 against 33.6 cycles per warp and step at four.
@@ -1129,16 +1132,16 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // `n_steps` steps of the warp's molecules.  With one molecule per thread they
   // go in groups without a look at the molecule in between (the bore test, the
   // step count and their branch otherwise sit on the step-to-step dependency
-  // chain: 229 instead of 260-290 cycles per step of a warp alone); a group in
-  // which the molecule ended is done again from its start, step by step.
+  // chain: 229 instead of 260-290 cycles per step of a warp alone).  A molecule
+  // that ends in a group is put back to the group's start and held; the held
+  // ones take their last steps together, one step at a time, every 64 steps (a
+  // warp of the defocusing lens ends one in a third of its groups, which taken
+  // again at once cost 20 runs of 1e7 molecules 12.23 instead of 11.69 ms).  A
+  // group that is to be taken again for another reason is at once.
   // sparse: few warps of the CTA have molecules, so the step's latency counts
   // and pieces are loaded ahead (lens_step_ahead), a group with a missed piece
-  // being done again as well; a warp that misses in more than half of its
-  // groups goes on without.  At 1024 threads (64 registers, 32 warps to hide
-  // latency) the linear form steps singly where the lens loses most molecules
-  // and groups are often done again: 8 runs of 3e6 molecules in the focusing
-  // lens 4.39 ms in groups, 4.89 singly; 20 runs of 1e7 in the defocusing one
-  // 13.20 and 13.13.
+  // being done again; a warp that misses in more than half of its groups goes
+  // on without.
   auto run = [&](const int n_steps, const bool sparse) {
     bool any = false;
 #pragma unroll
@@ -1148,14 +1151,17 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     if constexpr (kMPT == 1) {
       PersistSlot<M>& x = X[0];
       const float b = kSweep ? x.beta : L.beta;
-      // a group's steps by `advance` (true: all of them are the molecule's own)
+      // a group's steps by `advance`
       auto group = [&](auto&& advance) {
         constexpr int n = kRunGroup;
+        if (x.st.n_done + n > x.st.n_total) {
+          x.phase = kHold;
+          return;
+        }
         const float4 sa = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy), sb = make_float4(x.m.cx, x.m.cy, x.m.cvx, x.m.cvy);
-        bool ok = x.st.n_done + n <= x.st.n_total;
-        if constexpr (kRing) ok = ok && (!rec_on || x.to_rec > n);
-        if (ok) ok = advance();
-        if (ok) {
+        int how = kGroupAgain;
+        if (!kRing || !rec_on || x.to_rec > n) how = advance();
+        if (how == kGroupDone) {
           x.st.n_done += n;
           if constexpr (kRing) x.to_rec -= n;
           if (x.st.n_done == x.st.n_total) x.phase = kExit;
@@ -1168,10 +1174,22 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           x.m.cy = sb.y;
           x.m.cvx = sb.z;
           x.m.cvy = sb.w;
+          if (how == kGroupEnds) {
+            x.phase = kHold;
+          } else {
 #pragma unroll 1
-          for (int j = 0; j < n; ++j)
-            if (x.phase == kRun) step(x);
+            for (int j = 0; j < n; ++j)
+              if (x.phase == kRun) step(x);
+          }
         }
+      };
+      // the held molecules' last steps
+      auto release = [&]() {
+        if (!__any_sync(kFull, x.phase == kHold)) return;
+#pragma unroll 1
+        for (int j = 0; j < kRunGroup; ++j)
+          if (x.phase == kHold) step(x);
+        if (x.phase == kHold) x.phase = kRun;
       };
       // largest squared radius of the group within the bore; its distance is
       // the smallest of the group's, rounding being monotone
@@ -1192,6 +1210,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           unsigned missed = 0;
           for (; k + kRunGroup <= n_steps; k += kRunGroup) {
             if (k % 64 == 0) {
+              release();
               if (!__any_sync(kFull, x.phase == kRun)) return;
               if (__any_sync(kFull, missed > 64u / (2u * kRunGroup))) break;  // steps too wide to extrapolate
               missed = 0;
@@ -1206,28 +1225,30 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
                   r2max = fmaxf(r2max, r2);
                 }
                 missed += bad < 0x3f800000u ? 0u : 1u;
-                return bad < 0x3f800000u && inside(r2max);
+                return bad >= 0x3f800000u ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
               });
           }
         }
       }
-      if (kT < 1024 || F != kForceStark2Lin || !L.outward) {
-        for (; k + kRunGroup <= n_steps; k += kRunGroup) {
-          if (k % 64 == 0 && !__any_sync(kFull, x.phase == kRun)) return;
-          if (x.phase == kRun)
-            group([&]() {
-              float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
-              unsigned flags = 0;
-#pragma unroll
-              for (int j = 0; j < kRunGroup; ++j) {
-                x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
-                                                                      x.kappa);
-                r2max = fmaxf(r2max, r2);
-              }
-              return flags == 0 && inside(r2max);
-            });
+      for (; k + kRunGroup <= n_steps; k += kRunGroup) {
+        if (k % 64 == 0) {
+          release();
+          if (!__any_sync(kFull, x.phase == kRun)) return;
         }
+        if (x.phase == kRun)
+          group([&]() {
+            float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+            unsigned flags = 0;
+#pragma unroll
+            for (int j = 0; j < kRunGroup; ++j) {
+              x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
+                                                                    x.kappa);
+              r2max = fmaxf(r2max, r2);
+            }
+            return flags != 0 ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
+          });
       }
+      release();
     }
     while (k < n_steps) {
       const int stop = min(n_steps, k - k % 64 + 64);

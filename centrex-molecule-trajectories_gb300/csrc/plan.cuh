@@ -58,7 +58,6 @@ struct LensArgs {
   float bore2;  // (d/2)^2
   float bore;   // d/2
   int classic;
-  int outward;  // LensF::outward
   unsigned min_count, max_count;  // k_lens_persist, k_sweep_persist: queued molecules this launch takes
 };
 
@@ -101,7 +100,6 @@ __host__ __device__ inline LensArgs lens_args(const Plan& P, int li, bool staged
   a.bore2 = P.ef[li].c[0];
   a.bore = P.ef[li].c[1];
   a.classic = P.el[li].scheme == CTRAJ_RK4_CLASSIC;
-  a.outward = f.outward;
   a.min_count = 1u;
   a.max_count = 0xFFFFFFFFu;
   return a;
