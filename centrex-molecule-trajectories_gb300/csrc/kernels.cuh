@@ -885,6 +885,7 @@ static_assert(64 % kRunGroup == 0, "groups fill 64 steps");
 // What became of a group: its steps were the molecule's, they are to be taken
 // again one at a time, or the molecule ends among them.
 enum : int { kGroupDone, kGroupAgain, kGroupEnds };
+constexpr unsigned kThinLanes = 256, kThinRounds = 3;  // persist_pass
 // Phase B loads table pieces ahead while a CTA's molecules fill at most this
 // many warps: 176-212 cycles per step at one warp per scheduler against 229-264,
 // but 39.6 against 33.6 cycles per warp and step at four.
@@ -1309,6 +1310,17 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // shorter than that is dealt out molecule by molecule over the CTAs, each
   // CTA's share over as few warps per scheduler as hold it
   const bool short_queue = kMPT == 1 && static_entries > n_in;
+  // Where a lens loses most molecules and the queue is one to three rounds, the
+  // molecules that live longest end long after the others, and step slowest
+  // while the SM is full: an eighth of the CTAs starts with the first entries
+  // and eight warps only (317 instead of 538 cycles per step), so that these
+  // begin early.  1e7 molecules in the defocusing lens (2.05 rounds): 945 -> 919
+  // us, 5e6 721 -> 690.  With more rounds the lanes left empty cost what it gives.
+  unsigned thin = 0;
+  if (kT == kPersistThreads && kMPT == 1 && F == kForceStark2Lin && kStaged && !short_queue &&
+      n_in <= kThinRounds * static_entries && P.lf[li].outward)
+    thin = gridDim.x / 8u;
+  const unsigned dealt = static_entries - thin * (unsigned(kT) - kThinLanes);  // entries dealt out at first
   const unsigned share = blockIdx.x < n_in ? (n_in - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
   unsigned busy = kT / 32u;  // warps with molecules
   if (short_queue) {
@@ -1316,6 +1328,11 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     const unsigned per = busy ? (share + busy - 1u) / busy : 0u;  // of the CTA's share, in order: a warp's live alike
     const unsigned j = unsigned(warp) * per + unsigned(lane);
     if (unsigned(lane) < per && j < share) take(X[0], j * gridDim.x + blockIdx.x);
+  } else if (thin) {
+    const bool in = blockIdx.x < thin;
+    const unsigned j = in ? (unsigned(warp) * thin + blockIdx.x) * 32u + unsigned(lane)
+                          : thin * kThinLanes + (unsigned(warp) * (gridDim.x - thin) + blockIdx.x - thin) * 32u + unsigned(lane);
+    if (!in || unsigned(warp) < kThinLanes / 32u) take(X[0], j);
   } else {
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) {
@@ -1323,8 +1340,9 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
       if (j < min(n_in, static_entries)) take(X[s], j);
     }
   }
-  // phase A
-  for (bool exhausted = static_entries >= n_in && static_entries > 0; !exhausted;) {
+  // phase A (the further warps of a thin CTA wait at phase B's barrier)
+  const bool further = blockIdx.x < thin && unsigned(warp) >= kThinLanes / 32u;
+  for (bool exhausted = (dealt >= n_in && dealt > 0) || further; !exhausted;) {
     run(service, false);
     unsigned idle[kMPT], n_idle = 0;
 #pragma unroll
@@ -1336,7 +1354,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     if (n_idle) {
       unsigned b = 0;
       if (lane == 0) b = atomicAdd(Qin.head, n_idle);
-      b = static_entries + __shfl_sync(kFull, b, 0);
+      b = dealt + __shfl_sync(kFull, b, 0);
       exhausted = b + n_idle >= n_in;
 #pragma unroll
       for (int s = 0; s < kMPT; ++s) {
@@ -1345,7 +1363,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         b += unsigned(__popc(idle[s]));
       }
     } else {
-      exhausted = static_entries + *(volatile unsigned*)Qin.head >= n_in;
+      exhausted = dealt + *(volatile unsigned*)Qin.head >= n_in;
     }
   }
   // phase B (every warp of the CTA enters it, then the barriers below match):

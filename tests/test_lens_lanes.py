@@ -27,8 +27,9 @@ def _args(sigma):
     return compile_beamline(lens_beamline()), dict(xdist=xs, vdist=vs)
 
 
-# groups of four runs: queues of less than 1, of 1 to 8, of 8 to 32 and of more than 32 rounds of 512 lanes on 152 SMs
-@pytest.mark.parametrize("n", [10_001, 100_001, 250_001, 900_001])
+# groups of four runs: queues of less than 1, of 1 to 3 (some CTAs thin), of 3 to 8, of 8 to 32 and of more than 32 rounds
+# of 512 lanes on 152 SMs
+@pytest.mark.parametrize("n", [10_001, 19_470, 40_001, 57_001, 100_001, 250_001, 900_001])
 def test_batch_equals_single_runs(engine, n):
     cb, kw = _args(2.0)
     seeds = [3, 4, 5, 6]
