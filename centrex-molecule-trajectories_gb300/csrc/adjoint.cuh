@@ -895,8 +895,28 @@ __device__ __forceinline__ int soft_dropped_at(int k, int N) {
 // exp(-z) < 2^-54 and the log sigmoid and its derivative are -e and e to the
 // last bit).  Every value is k_soft_lens's, the sums in its order.
 // Up to kQuad64Max queued molecules and checkpoint intervals of whole eights;
-// 1e4 molecules (270 queued), gradient: 22.2 -> 7.5 ms.
-template <bool kGrad>
+// 1e4 molecules (270 queued), gradient: 22.2 -> 7.5 ms, with kSplit 4.8.
+// kSplit: warps 0 and 1 of a CTA take the steps and warps 2 and 3, on the
+// schedulers that would be idle, the tests of their states, eight steps behind
+// through shared memory: 32 instead of 40 to 49 FP64 instructions per step on
+// the steps' chain.  For up to two eights of molecules per SM, where every
+// stepping warp has its scheduler to itself; beyond, the pipes are all busy.
+// The two warps of a pair meet at a named barrier after every block of eight
+// steps; both know the blocks of their molecules (the largest step count) and
+// after the barrier of block k whether a molecule was left at the tests of
+// block k - 1, so both leave at the same one.
+constexpr size_t kSoftSmem = 227 * 1024;  // shared memory of a CTA
+constexpr int kQuadBlock = 8;
+struct QuadShared {
+  double state[2][2][kQuadBlock][8][2];  // pair, parity of the block, step, molecule, component
+  double last[2][8][8];                  // pair, (x, y, vx, vy, cx, cy, cvx, cvy), molecule
+  int live[2][2];                        // pair, parity of the block: molecules left after its tests
+};
+__device__ __forceinline__ void pair_sync(int pair) {
+  asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+}
+
+template <bool kGrad, bool kSplit>
 __global__ void __launch_bounds__(kSoftThreads) k_soft_lens_quad(const __grid_constant__ SoftPlan S, const SoftQueue Q,
                                                                  const Coef4<double>* __restrict__ table, double* ckpt,
                                                                  size_t cap, double* __restrict__ contrib,
@@ -905,16 +925,18 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens_quad(const __grid_co
   Coef4<double>* s_tab = reinterpret_cast<Coef4<double>*>(s_raw);
   stage_table(S, table, s_tab);
   const unsigned n_in = Q.size();
-  const int lane = threadIdx.x & 31, part = lane & 3, home = lane & ~3;
+  const int lane = threadIdx.x & 31, part = lane & 3, home = lane & ~3, mol = lane >> 2, warp = threadIdx.x >> 5;
   const bool half = part & 2;
+  const int pair = warp & 1;
+  const bool stepper = !kSplit || warp < 2;
   const double inv_w = S.inv_w, bore = S.bore, floor_ = S.log_floor;
   const SoftK<double> C(S);
   const double g = (part & 1) ? -C.g : -0.0;  // a + (-0.0) is a
   const int K = S.checkpoint;
   unsigned long long steps = 0, dropped = 0, entered = 0;
-  const unsigned batches = (n_in + 7u) / 8u, warps = gridDim.x * (blockDim.x / 32u);
-  for (unsigned b = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; b < batches; b += warps) {
-    const unsigned slot = b * 8u + unsigned(lane >> 2);
+  const unsigned batches = (n_in + 7u) / 8u, warps = gridDim.x * (kSplit ? 2u : blockDim.x / 32u);
+  for (unsigned b = unsigned(kSplit ? pair : warp) * gridDim.x + blockIdx.x; b < batches; b += warps) {
+    const unsigned slot = b * 8u + unsigned(mol);
     const bool have = slot < n_in;
     const int64_t i = Q.at(have ? slot : 0u);  // lanes beyond the queue repeat a molecule and store nothing
     SoftMol<double> m;
@@ -937,38 +959,30 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens_quad(const __grid_co
       const Coef4<double> q = s_tab[j];
       return fma_(mul_(C.kappa, fma_(u, fma_(u, q.q2, q.q1), q.q0)), p, g);
     };
-    for (int n = 0; __any_sync(kFull, n < N && below < 0); n += 4) {
-      if (kGrad && n % K == 0 && n < N && below < 0) {
-        double* o = ckpt + size_t(n / K) * 8 * cap + slot;
-        o[size_t(part) * cap] = half ? V : X;
-        o[size_t(4 + part) * cap] = c;
+    auto step = [&](const bool run) {
+      const double l12 = force(half ? fma_(L.c2, V, X) : X);
+      const double l34 = force(fma_(c34, fma_(L.hdt, l12, V), X));
+      const double m12 = __shfl_xor_sync(kFull, l12, 2), m34 = __shfl_xor_sync(kFull, l34, 2);
+      // halves: (l1 + l2) + l3 -> dt26 (.) + dt v | 2 (l2 + l3) + (l1 + l4) -> dt6 (.)
+      const double a = add_(l12, half ? m34 : m12), e = add_(half ? m12 : a, l34);
+      const double f = fma_(half ? 2.0 : L.dt, half ? a : V, half ? e : -0.0);
+      const double inc = fma_(half ? L.dt6 : L.dt26, half ? f : e, half ? -0.0 : f);
+      const double s0 = half ? V : X, d = add_(inc, c), t = add_(s0, d);
+      const double err = add_(d, -add_(t, -s0));
+      const double o = __shfl_xor_sync(kFull, t, 2);
+      if (run) {
+        X = half ? o : t;
+        V = half ? t : o;
+        c = err;
       }
-      double qx = 0.0, qy = 0.0;  // this lane's state to test: after step n + part
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        const bool run = n + j < N;
-        const double l12 = force(half ? fma_(L.c2, V, X) : X);
-        const double l34 = force(fma_(c34, fma_(L.hdt, l12, V), X));
-        const double m12 = __shfl_xor_sync(kFull, l12, 2), m34 = __shfl_xor_sync(kFull, l34, 2);
-        // halves: (l1 + l2) + l3 -> dt26 (.) + dt v | 2 (l2 + l3) + (l1 + l4) -> dt6 (.)
-        const double a = add_(l12, half ? m34 : m12), e = add_(half ? m12 : a, l34);
-        const double f = fma_(half ? 2.0 : L.dt, half ? a : V, half ? e : -0.0);
-        const double inc = fma_(half ? L.dt6 : L.dt26, half ? f : e, half ? -0.0 : f);
-        const double s0 = half ? V : X, d = add_(inc, c), t = add_(s0, d);
-        const double err = add_(d, -add_(t, -s0));
-        const double o = __shfl_xor_sync(kFull, t, 2);
-        if (run) {
-          X = half ? o : t;
-          V = half ? t : o;
-          c = err;
-        }
-        const double tx = __shfl_sync(kFull, X, home), ty = __shfl_sync(kFull, X, home + 1);
-        if (part == j) {
-          qx = tx;
-          qy = ty;
-        }
-      }
-      // the four states' tests, added in step order
+    };
+    auto store_ckpt = [&](const int n) {
+      double* o = ckpt + size_t(n / K) * 8 * cap + slot;
+      o[size_t(part) * cap] = half ? V : X;
+      o[size_t(4 + part) * cap] = c;
+    };
+    // the tests of the states after steps n .. n + 3, (qx, qy) this lane's, added in step order
+    auto tests = [&](const int n, const double qx, const double qy) {
       const bool use = n + part < N;
       const double r2 = fma_(qy, qy, mul_(qx, qx));
       double h;
@@ -990,6 +1004,57 @@ __global__ void __launch_bounds__(kSoftThreads) k_soft_lens_quad(const __grid_co
         m.lw = add_(m.lw, __shfl_sync(kFull, ls, home + j));
         m.d_bore = add_(m.d_bore, __shfl_sync(kFull, dr, home + j));
         if (below < 0 && n + j < N && !(m.lw >= floor_)) below = n + j + 1;
+      }
+    };
+    if constexpr (kSplit) {
+      QuadShared& H = *reinterpret_cast<QuadShared*>(s_tab + S.n_int);  // behind the table
+      const int blocks = (__reduce_max_sync(kFull, N) + kQuadBlock - 1) / kQuadBlock;
+      pair_sync(pair);  // the tests' warp has read the last batch's states
+      for (int k = 0; k < blocks; ++k) {
+        const int n = k * kQuadBlock;
+        if (stepper) {
+          if (kGrad && n % K == 0 && n < N) store_ckpt(n);
+#pragma unroll 1
+          for (int j = 0; j < kQuadBlock; ++j) {
+            step(n + j < N);
+            if (!half) H.state[pair][k & 1][j][mol][part] = X;
+          }
+        }
+        pair_sync(pair);
+        if (k > 0 && !H.live[pair][(k - 1) & 1]) break;
+        if (!stepper) {
+#pragma unroll 1
+          for (int j = 0; j < kQuadBlock; j += 4) {
+            const double* q = H.state[pair][k & 1][j + part][mol];
+            tests(n + j, q[0], q[1]);
+          }
+          const bool left = __any_sync(kFull, n + kQuadBlock < N && below < 0);
+          if (lane == 0) H.live[pair][k & 1] = left;
+        }
+      }
+      if (stepper) {
+        H.last[pair][part][mol] = half ? V : X;
+        H.last[pair][4 + part][mol] = c;
+      }
+      pair_sync(pair);
+      if (stepper) continue;
+      X = H.last[pair][part & 1][mol];
+      V = H.last[pair][2 + (part & 1)][mol];
+      c = H.last[pair][4 + part][mol];
+    } else {
+      for (int n = 0; __any_sync(kFull, n < N && below < 0); n += 4) {
+        if (kGrad && n % K == 0 && n < N && below < 0) store_ckpt(n);
+        double qx = 0.0, qy = 0.0;  // this lane's state to test: after step n + part
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          step(n + j < N);
+          const double tx = __shfl_sync(kFull, X, home), ty = __shfl_sync(kFull, X, home + 1);
+          if (part == j) {
+            qx = tx;
+            qy = ty;
+          }
+        }
+        tests(n, qx, qy);
       }
     }
     const double x = __shfl_sync(kFull, X, home), y = __shfl_sync(kFull, X, home + 1);

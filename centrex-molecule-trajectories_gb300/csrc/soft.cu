@@ -204,10 +204,15 @@ int soft_run(ctraj_context* c, const ctraj_soft_args* a, SoftPlan& S, int li, ct
       if constexpr (std::is_same<T, double>::value) {
         quad = count <= kQuad64Max && S.checkpoint % 8 == 0;
         if (quad) {
-          auto kq = a->want_grad ? k_soft_lens_quad<true> : k_soft_lens_quad<false>;
-          CT_CUDA(cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tb)));
+          const unsigned batches = (count + 7u) / 8u;
+          // a scheduler for every warp, and room beside the table
+          const bool split = batches <= 2u * unsigned(c->sm_count) && tb + sizeof(QuadShared) <= kSoftSmem;
+          const size_t qb = tb + (split ? sizeof(QuadShared) : 0);
+          auto kq = a->want_grad ? (split ? k_soft_lens_quad<true, true> : k_soft_lens_quad<true, false>)
+                                 : (split ? k_soft_lens_quad<false, true> : k_soft_lens_quad<false, false>);
+          CT_CUDA(cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, int(qb)));
           // eight molecules per warp, a warp per CTA while there are SMs
-          kq<<<std::min((count + 7u) / 8u, unsigned(c->sm_count)), kSoftThreads, tb, s>>>(
+          kq<<<std::min(batches, unsigned(c->sm_count)), kSoftThreads, qb, s>>>(
               S, Q, c->soft_table.as<Coef4<T>>(), c->soft_ckpt.as<T>(), cap, contrib, stats);
         }
       }

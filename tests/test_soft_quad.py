@@ -58,3 +58,34 @@ def test_the_lens_pass_edge_test_is_the_general_one(radius, inv_w):
     bad = ctypes.c_ulonglong(1)
     assert lib.ctraj_peak_soft_test_check(radius, inv_w, ctypes.byref(bad)) == 0
     assert bad.value == 0
+
+
+# queues whose tests have warps of their own (up to two eights of molecules per SM) against one that has not: one
+# molecule, an incomplete eight, the last such queue, and step counts that are not whole blocks (dt)
+@pytest.mark.parametrize("low,dt_scale,part", [(False, 1.0, 20_000), (True, 1.0, 40_000), (True, 7.3, 13_337), (False, 3.1, 84_000)])
+def test_tests_in_their_own_warps(low, dt_scale, part):
+    from ctraj.adjoint import SoftProblem, soft_transmission
+    from ctraj.engine import Engine
+    from ctraj.workloads import lens_beamline
+
+    bl = lens_beamline(V=10e3 if low else 30e3, low_field_seeker=low, detector_d=12e-3)
+    bl.elements[1].dt *= dt_scale
+    eng = Engine(0)
+
+    def run(n, offset, grad=True):
+        prob = SoftProblem.from_beamline(bl, n=n, aperture="A1", precision=64, seed=8, offset=offset)
+        return soft_transmission(prob, prob.initial_params(), want_grad=grad, engine=eng)
+
+    try:
+        k = 240_000 // part
+        whole, parts = run(k * part, 0), [run(part, j * part) for j in range(k)]
+        assert 2_432 < whole.lens_molecules <= 10_000 and max(p.lens_molecules for p in parts) <= 2_432
+        for f in ("lens_molecules", "lens_steps", "dropped"):
+            assert sum(getattr(p, f) for p in parts) == getattr(whole, f), f
+        assert abs(sum(p.loss for p in parts) / k - whole.loss) <= 1e-13 * whole.loss
+        g = sum(p.grad for p in parts) / k
+        assert np.abs(g - whole.grad).max() <= 1e-11 * np.abs(whole.grad).max()
+        a, b = run(37, 0), run(37, 0, grad=False)  # about one molecule in the queue
+        assert a.loss == b.loss and (a.lens_steps, a.dropped) == (b.lens_steps, b.dropped)
+    finally:
+        eng.close()
