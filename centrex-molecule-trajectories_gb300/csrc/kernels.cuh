@@ -1116,17 +1116,21 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     derive(x);
     x.phase = !ok ? kBad : (x.st.n_done < x.st.n_total ? kRun : kExit);
   };
+  // the state after step n (counted from the entrance), when the record takes it
+  auto record = [&](PersistSlot<M>& x, const int n) {
+    if constexpr (kRing) {
+      if (rec_on && --x.to_rec == 0) {
+        x.to_rec = R.rec_stride;
+        R.rec[size_t(x.cfg) * R.rec_max + n / R.rec_stride] = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy);
+      }
+    }
+  };
   auto step = [&](PersistSlot<M>& x) {
     bool lost = x.m.template lens_step<F, kStaged, kSweep>(L, x.dt, x.hdt, x.c2, x.dt6, x.dt26, s_tab, x.flags,
                                                           x.beta, x.kappa);
     if (F == kForceRadial && (x.flags & 2u)) lost = true;
     ++x.st.n_done;
-    if constexpr (kRing) {
-      if (rec_on && --x.to_rec == 0) {
-        x.to_rec = R.rec_stride;
-        R.rec[size_t(x.cfg) * R.rec_max + x.st.n_done / R.rec_stride] = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy);
-      }
-    }
+    record(x, x.st.n_done);
     if (lost) x.phase = kLost;
     else if (x.st.n_done == x.st.n_total) x.phase = kExit;
   };
@@ -1138,7 +1142,11 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // ones take their last steps together, one step at a time, every 64 steps (a
   // warp of the defocusing lens ends one in a third of its groups, which taken
   // again at once cost 20 runs of 1e7 molecules 12.23 instead of 11.69 ms).  A
-  // group that is to be taken again for another reason is at once.
+  // group that is to be taken again for another reason is at once.  Ring
+  // recording stores the states of a group as it goes (those after an end are
+  // behind the record's last row, those of a group taken again stored again;
+  // 1.25e8 molecules recorded every 50 steps: 10.4 ms, 15.3 with such groups
+  // taken singly).
   // sparse: few warps of the CTA have molecules, so the step's latency counts
   // and pieces are loaded ahead (lens_step_ahead), a group with a missed piece
   // being done again; a warp that misses in more than half of its groups goes
@@ -1160,11 +1168,10 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           return;
         }
         const float4 sa = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy), sb = make_float4(x.m.cx, x.m.cy, x.m.cvx, x.m.cvy);
-        int how = kGroupAgain;
-        if (!kRing || !rec_on || x.to_rec > n) how = advance();
+        const int to_rec = x.to_rec;
+        const int how = advance();
         if (how == kGroupDone) {
           x.st.n_done += n;
-          if constexpr (kRing) x.to_rec -= n;
           if (x.st.n_done == x.st.n_total) x.phase = kExit;
         } else {
           x.m.x = sa.x;
@@ -1175,6 +1182,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           x.m.cy = sb.y;
           x.m.cvx = sb.z;
           x.m.cvy = sb.w;
+          if constexpr (kRing) x.to_rec = to_rec;
           if (how == kGroupEnds) {
             x.phase = kHold;
           } else {
@@ -1224,6 +1232,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
                 for (int j = 0; j < kRunGroup; ++j) {
                   x.m.template lens_step_ahead<kSweep>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, q, r2, bad, b, x.kappa);
                   r2max = fmaxf(r2max, r2);
+                  record(x, x.st.n_done + j + 1);
                 }
                 missed += bad < 0x3f800000u ? 0u : 1u;
                 return bad >= 0x3f800000u ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
@@ -1245,6 +1254,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
               x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
                                                                     x.kappa);
               r2max = fmaxf(r2max, r2);
+              record(x, x.st.n_done + j + 1);
             }
             return flags != 0 ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
           });
