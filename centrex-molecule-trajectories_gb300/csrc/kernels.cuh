@@ -1134,7 +1134,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     if (lost) x.phase = kLost;
     else if (x.st.n_done == x.st.n_total) x.phase = kExit;
   };
-  // `n_steps` steps of the warp's molecules.  With one molecule per thread they
+  // `n_steps` steps of the warp's molecules, a thread's one after the other.  They
   // go in groups without a look at the molecule in between (the bore test, the
   // step count and their branch otherwise sit on the step-to-step dependency
   // chain: 229 instead of 260-290 cycles per step of a warp alone).  A molecule
@@ -1157,11 +1157,9 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     for (int s = 0; s < kMPT; ++s) any = any || X[s].phase == kRun;
     if (!__any_sync(kFull, any)) return;
     int k = 0;
-    if constexpr (kMPT == 1) {
-      PersistSlot<M>& x = X[0];
-      const float b = kSweep ? x.beta : L.beta;
+    {
       // a group's steps by `advance`
-      auto group = [&](auto&& advance) {
+      auto group = [&](PersistSlot<M>& x, auto&& advance) {
         constexpr int n = kRunGroup;
         if (x.st.n_done + n > x.st.n_total) {
           x.phase = kHold;
@@ -1193,7 +1191,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         }
       };
       // the held molecules' last steps
-      auto release = [&]() {
+      auto release = [&](PersistSlot<M>& x) {
         if (!__any_sync(kFull, x.phase == kHold)) return;
 #pragma unroll 1
         for (int j = 0; j < kRunGroup; ++j)
@@ -1202,7 +1200,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
       };
       // largest squared radius of the group within the bore; its distance is
       // the smallest of the group's, rounding being monotone
-      auto inside = [&](const float r2max) {
+      auto inside = [&](PersistSlot<M>& x, const float r2max) {
         if (!(r2max <= L.bore2)) return false;
         if constexpr (kOut) {
           const float d = __fadd_rn(sqrtf(r2max), -L.bore);
@@ -1212,20 +1210,22 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         return true;
       };
       const PairTable T = pair_table<F>(L, kStaged ? s_tab : L.q);
-      if constexpr (F == kForceStark2Lin && kStaged) {
+      if constexpr (F == kForceStark2Lin && kStaged && kMPT == 1) {
         if (sparse) {
+          PersistSlot<M>& x = X[0];
+          const float b = kSweep ? x.beta : L.beta;
           LinAhead q;
           q.clear();
           unsigned missed = 0;
           for (; k + kRunGroup <= n_steps; k += kRunGroup) {
             if (k % 64 == 0) {
-              release();
+              release(x);
               if (!__any_sync(kFull, x.phase == kRun)) return;
               if (__any_sync(kFull, missed > 64u / (2u * kRunGroup))) break;  // steps too wide to extrapolate
               missed = 0;
             }
             if (x.phase == kRun)
-              group([&]() {
+              group(x, [&]() {
                 float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
                 unsigned bad = 0;
 #pragma unroll
@@ -1235,31 +1235,42 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
                   record(x, x.st.n_done + j + 1);
                 }
                 missed += bad < 0x3f800000u ? 0u : 1u;
-                return bad >= 0x3f800000u ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
+                return bad >= 0x3f800000u ? kGroupAgain : inside(x, r2max) ? kGroupDone : kGroupEnds;
               });
           }
         }
       }
       for (; k + kRunGroup <= n_steps; k += kRunGroup) {
         if (k % 64 == 0) {
-          release();
-          if (!__any_sync(kFull, x.phase == kRun)) return;
-        }
-        if (x.phase == kRun)
-          group([&]() {
-            float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
-            unsigned flags = 0;
+          any = false;
 #pragma unroll
-            for (int j = 0; j < kRunGroup; ++j) {
-              x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
-                                                                    x.kappa);
-              r2max = fmaxf(r2max, r2);
-              record(x, x.st.n_done + j + 1);
-            }
-            return flags != 0 ? kGroupAgain : inside(r2max) ? kGroupDone : kGroupEnds;
-          });
+          for (int s = 0; s < kMPT; ++s) {
+            release(X[s]);
+            any = any || X[s].phase == kRun;
+          }
+          if (!__any_sync(kFull, any)) return;
+        }
+#pragma unroll
+        for (int s = 0; s < kMPT; ++s) {
+          PersistSlot<M>& x = X[s];
+          if (x.phase == kRun)
+            group(x, [&]() {
+              const float b = kSweep ? x.beta : L.beta;
+              float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+              unsigned flags = 0;
+#pragma unroll
+              for (int j = 0; j < kRunGroup; ++j) {
+                x.m.template lens_step_pair<F, kStaged, kSweep, true>(L, T, x.dt, x.hdt, x.c2, x.dt6, x.dt26, r2, flags, b,
+                                                                      x.kappa);
+                r2max = fmaxf(r2max, r2);
+                record(x, x.st.n_done + j + 1);
+              }
+              return flags != 0 ? kGroupAgain : inside(x, r2max) ? kGroupDone : kGroupEnds;
+            });
+        }
       }
-      release();
+#pragma unroll
+      for (int s = 0; s < kMPT; ++s) release(X[s]);
     }
     while (k < n_steps) {
       const int stop = min(n_steps, k - k % 64 + 64);
