@@ -1111,6 +1111,8 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     if (x.fresh) {  // step setup deferred by the front kernel
       x.m.load_vz(Qin, x.idx);
       ok = enter_lens(x.m, P, li, x.st);
+    } else {
+      x.st.snap = double(Qin.snap[x.idx]);  // of a second lens; a deferred end takes it from here
     }
     x.n0 = x.st.n_done;
     derive(x);
