@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "fp64.cuh"
 #include "philox.cuh"
 #include "plan.cuh"
 
@@ -499,21 +500,35 @@ struct Mol64 {
     if (kRec) sink->write(x[0], x[1], x[2], v[0], v[1], v[2], a[0], a[1], a[2], t);
   }
 
-  // Molecule.update_trajectory(delta_t, a=(0,-g,0))
+  // Molecule.update_trajectory(delta_t, a=(0,-g,0)).  In a flight with a_x and
+  // a_z zero their terms are +0 or -0, which change a sum only where it is -0
+  // itself: 22 FP64 instructions instead of 35 (with the tests on the integer
+  // pipe; front of 1e5 ballistic molecules 35.7 -> 29.5 us), all of them for
+  // other accelerations and for numbers whose products could leave the normal
+  // range.
   __device__ void update(double dt, const Plan& P) {
-    if (dt != 0.0) {  // `if not delta_t` keeps x and v (molecule.py:31,41)
+    if (!is_zero(dt)) {  // `if not delta_t` keeps x and v (molecule.py:31,41)
       const double dt2 = dmul(dt, dt);
+      if (__double_as_longlong(a[0]) == 0 && __double_as_longlong(a[2]) == 0 && in_range<-200, 200>(dt) &&
+          in_range<-200, 200>(a[1]) && !is_zero(v[0]) && !is_zero(v[2])) {
+        const double sx = dadd(x[0], dmul(v[0], dt)), sz = dadd(x[2], dmul(v[2], dt));
+        x[0] = is_zero(sx) ? 0.0 : sx;
+        x[2] = is_zero(sz) ? 0.0 : sz;
+        x[1] = dadd(dadd(x[1], dmul(v[1], dt)), dmul(scale2(a[1], -1), dt2));
+        v[1] = dadd(v[1], dmul(a[1], dt));
+      } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        x[k] = dadd(dadd(x[k], dmul(v[k], dt)), dmul(dmul(a[k], dt2), 0.5));
-        v[k] = dadd(v[k], dmul(a[k], dt));
+        for (int k = 0; k < 3; ++k) {
+          x[k] = dadd(dadd(x[k], dmul(v[k], dt)), dmul(dmul(a[k], dt2), 0.5));
+          v[k] = dadd(v[k], dmul(a[k], dt));
+        }
       }
     }
     t = dadd(t, dt);
     a[0] = 0.0;
     a[1] = -P.g;
     a[2] = 0.0;
-    rows += isfinite(t) ? 1 : 0;
+    rows += (hi_word(t) & 0x7ff00000) != 0x7ff00000 ? 1 : 0;  // finite
     row_out();
   }
 
