@@ -1201,10 +1201,14 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
         if (x.phase == kHold) x.phase = kRun;
       };
       // largest squared radius of the group within the bore; its distance is
-      // the smallest of the group's, rounding being monotone
+      // the smallest of the group's, rounding being monotone.  kNoRadius: every
+      // one of the group is NaN (fmaxf leaves a NaN out), which is not lost and
+      // has no distance to note, as in a step looked at by itself.
+      constexpr float kNoRadius = -1.0f;
       auto inside = [&](PersistSlot<M>& x, const float r2max) {
         if (!(r2max <= L.bore2)) return false;
         if constexpr (kOut) {
+          if (r2max == kNoRadius) return true;
           const float d = __fadd_rn(sqrtf(r2max), -L.bore);
           if (d > 0.0f) return false;
           x.m.note(d);
@@ -1228,7 +1232,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
             }
             if (x.phase == kRun)
               group(x, [&]() {
-                float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+                float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = kNoRadius;
                 unsigned bad = 0;
 #pragma unroll
                 for (int j = 0; j < kRunGroup; ++j) {
@@ -1258,7 +1262,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           if (x.phase == kRun)
             group(x, [&]() {
               const float b = kSweep ? x.beta : L.beta;
-              float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = 0.0f;
+              float r2 = __fmaf_rn(x.m.y, x.m.y, __fmul_rn(x.m.x, x.m.x)), r2max = kNoRadius;
               unsigned flags = 0;
 #pragma unroll
               for (int j = 0; j < kRunGroup; ++j) {
