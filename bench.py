@@ -118,12 +118,13 @@ def parse():
                    help="--profile lens/sweep: the FP32 lens pass to run (ctraj_tuning.lens_mode)")
     p.add_argument("--batch-group", type=int, default=10, help="--profile batch: runs per shared lens pass")
     p.add_argument("--front-threads", type=int, default=128, help="--profile: threads per front block")
-    p.add_argument("--batch-lens-threads", type=int, default=1024,
-                   help="--profile batch: threads per CTA of the shared lens pass")
+    p.add_argument("--batch-lens-threads", type=int, default=0,
+                   help="--profile batch: threads per CTA of the shared lens pass (0: by the queue's length)")
     p.add_argument("--lens-interval", type=int, default=256,
                    help="--profile: RK4 steps between the persistent pass's compactions once its queue is empty")
-    p.add_argument("--lens-threads", type=int, default=512,
-                   help="--profile lens/sweep: threads per CTA of a run's or a sweep's persistent lens pass")
+    p.add_argument("--lens-threads", type=int, default=0,
+                   help="--profile lens/sweep: threads per CTA of a run's or a sweep's persistent lens pass "
+                        "(0: by the queue's length)")
     return p.parse_args()
 
 
@@ -886,7 +887,8 @@ def main():
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     roofline = {"bound": "fp32",
                 "kernel": f"k_lens_persist, grouped: the lens pass {tun['batch_group']} runs of the batch share "
-                          f"({tun['batch_lens_threads']} threads per CTA, one CTA per SM; with its entrant "
+                          f"({tun['batch_lens_threads'] or 'by the queue 512, 768 or 1024'} threads per CTA, one CTA "
+                          f"per SM; with its entrant "
                           f"ordering and k_lens_finish, timed together)",
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                 "peak_source": "measured in this run: FMA-chain kernel (bench_kernels/fp32_peak.cu), "

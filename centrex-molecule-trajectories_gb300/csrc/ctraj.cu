@@ -297,7 +297,7 @@ constexpr unsigned kWideRounds = 8, kWidestRounds = 32, kWideShare = 32;
 
 int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i, const Queue& Qin,
                        const Queue& Qnext, unsigned* order_buf, int sms, int interval, int service, cudaStream_t s,
-                       int* launches, int lanes, int mpt, DoneRec* done, unsigned by_count) {
+                       int* launches, int lanes, int mpt, DoneRec* done, unsigned most) {
   const bool staged = P.lf[i].n_smem > 0;
   unsigned* hist = order_buf;
   unsigned* order = hist + kOrderBuckets;
@@ -326,26 +326,31 @@ int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i
   // a step's latency; with 512 a molecule's own steps are faster, which is what
   // a short queue waits for.  Linear form: 768 over 512 lanes at 2.8, 7, 17 and
   // 69 rounds 1.06, 1.02, 0.92 and 0.91 of the time; 1024 over 768 1.10, 1.08,
-  // 1.03 and 0.99.  A pass without a count rule takes the lanes it is given
-  // beyond one round (8 runs of 3e5 molecules in groups of 4, 20 000 entrants:
-  // 1.41 ms at 1024 lanes, 1.19 at 512).
+  // 1.03 and 0.99.  The other staged forms' batch passes have a second launch
+  // for one round only (8 runs of 3e5 molecules in groups of 4, 20 000
+  // entrants: 1.41 ms at 1024 lanes, 1.19 at 512).
   const unsigned round = unsigned(sms) * unsigned(kPersistThreads);
   const unsigned wide = kWideRounds * round, widest = kWidestRounds * round;
+  const bool batch = mode == kModeBatch;
+  const bool choose = lanes == 0 && mpt == 1 && staged && !out && mode != kModeRing;
   int st = CTRAJ_OK;
-  if (by_count && mpt == 1 && staged && !out && P.lf[i].force == kForceStark2Lin) {
-    // A pass that returns costs 4 us: a single run's are launched for a queue
-    // that a share of its molecules may fill, its queue being a few percent of
-    // them; a group's, whose queue is a whole group's, for one that all may.
-    const unsigned most = mode == kModeBatch ? by_count : by_count / kWideShare;
-    const bool any_wide = most > wide, any_widest = most > widest;
+  if (choose && P.lf[i].force == kForceStark2Lin) {
+    // A pass that returns costs 4 us (0.4 % of a run of 1e7 molecules, 0.7 % of
+    // one of 1e6): a single run's wider ones are launched where a 32nd of its
+    // molecules could need them, its queue being a few percent of them where an
+    // aperture stands before the lens; a group's, whose queue is a whole
+    // group's, where all of them could.  A single run most of whose molecules
+    // enter the lens so takes 512 lanes up to 32 times those queues.
+    const unsigned may = batch ? most : most / kWideShare;
+    const bool any_wide = may > wide, any_widest = may > widest;
     st = pass(kPersistThreads, 1, 1u, any_wide ? wide : 0xFFFFFFFFu);
     if (!st && any_wide) st = pass(768, 1, wide + 1u, any_widest ? widest : 0xFFFFFFFFu);
     if (!st && any_widest) st = pass(1024, 1, widest + 1u, 0xFFFFFFFFu);
-  } else if (lanes > kPersistThreads && mpt == 1) {
+  } else if (choose && batch) {
     st = pass(kPersistThreads, 1, 1u, round);
-    if (!st) st = pass(lanes, mpt, round + 1u, 0xFFFFFFFFu);
+    if (!st) st = pass(kBatchLensThreads, 1, round + 1u, 0xFFFFFFFFu);
   } else {
-    st = pass(lanes, mpt, 1u, 0xFFFFFFFFu);
+    st = pass(lanes ? lanes : batch ? kBatchLensThreads : kPersistThreads, mpt, 1u, 0xFFFFFFFFu);
   }
   if (st) return st;
   if (done) {  // the molecules' ends, in full warps
@@ -436,13 +441,10 @@ int launch_persistent(ctraj_context* c, bool out, int mode, const Plan& P, const
     if ((st = c->lens_done.ensure(size_t(count) * kDoneRecBytes, 25))) return st;
     done = c->lens_done.as<DoneRec>();
   }
-  // the tuning's default lanes: by the queue's length
-  const bool batch = mode == kModeBatch;
-  const int lanes = batch ? c->batch_lens_threads : c->lens_threads;
-  const bool by_count = (batch || mode == kModePlain) && lanes == (batch ? kBatchLensThreads : kPersistThreads);
+  const int lanes = mode == kModeBatch ? c->batch_lens_threads : c->lens_threads;
   return enqueue_persistent(out, mode, P, R, i, Qin, Qnext, c->lens_order.as<unsigned>(), c->sm_count,
                             c->lens_interval, c->lens_service, c->stream, launches, lanes, c->lens_molecules, done,
-                            by_count ? count : 0u);
+                            count);
 }
 
 // k_front, then for each lens: read the lens queue's size and largest
@@ -699,9 +701,10 @@ int ctraj_set_tuning(ctraj_context* c, const ctraj_tuning* t) {
       (t->lens_mode != CTRAJ_LENS_PERSISTENT && t->lens_mode != CTRAJ_LENS_CHUNKED) || t->lens_interval < 1 ||
       t->lens_interval > 100000 || (t->front_threads != 128 && t->front_threads != 256 && t->front_threads != 512) ||
       t->batch_group < 1 || t->batch_group > CTRAJ_MAX_BATCH_GROUP ||
-      (t->lens_threads != 512 && t->lens_threads != 768 && t->lens_threads != 1024) ||
+      (t->lens_threads != 0 && t->lens_threads != 512 && t->lens_threads != 768 && t->lens_threads != 1024) ||
       (t->lens_molecules != 1 && t->lens_molecules != 2) ||
-      (t->batch_lens_threads != 512 && t->batch_lens_threads != 768 && t->batch_lens_threads != 1024) ||
+      (t->batch_lens_threads != 0 && t->batch_lens_threads != 512 && t->batch_lens_threads != 768 &&
+       t->batch_lens_threads != 1024) ||
       t->lens_service < 1 || t->lens_service > 100000)
     return fail(CTRAJ_EINVAL,
                 "tuning out of range (chunk_first %d, chunk_growth %d, chunk_max %d, front_waves %d, lens_mode %d, "

@@ -78,7 +78,7 @@ struct HostTable {
 
 }  // namespace ctraj
 
-constexpr int kBatchLensThreads = 1024;  // default of batch_lens_threads
+constexpr int kBatchLensThreads = 1024;  // lanes of a batch group's lens passes that are not chosen by the queue
 
 // One context (ctraj_create): its device, stream, beamline, tables, tuning
 // and work buffers.
@@ -121,9 +121,9 @@ struct ctraj_context {
   int lens_service = 64;        // persistent mode: steps between a warp's refills (kPersistService)
   int front_threads = 256;      // k_front block size
   int batch_group = 4;          // ctraj_run_batch: runs sharing one lens pass
-  int lens_threads = 512;       // persistent FP32 lens pass: molecule lanes per CTA
+  int lens_threads = 0;         // persistent FP32 lens pass: molecule lanes per CTA, 0: by the queue's length
   int lens_molecules = 1;       // persistent FP32 lens pass: molecules per thread
-  int batch_lens_threads = kBatchLensThreads;  // lens_threads of a batch group's shared lens passes
+  int batch_lens_threads = 0;   // lens_threads of a batch group's shared lens passes
   unsigned run_max_steps = 0;   // largest lens queue step bound of the last run
   bool timing = false;
   // before front, after front, before the first lens chunk, after the last one
@@ -266,11 +266,11 @@ constexpr size_t kDoneRecBytes = 64;
 // queue's entries), then one k_lens_persist launch, one CTA per SM.  With
 // `done` (kDoneRecBytes per queue entry; plain or batch passes without
 // per-molecule outputs) the molecules' ends are deferred to one k_lens_finish
-// launch after the pass.  by_count: the most entries Qin can hold when the
-// lanes of the linear form are to be chosen by its count (on the device: the
-// passes that it does not suit return at once), else 0.
+// launch after the pass.  lanes 0: by Qin's count, of which the host knows only
+// the most it can be (on the device: the passes that it does not suit return at
+// once); other lanes are taken as given.
 int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i, const Queue& Qin,
                        const Queue& Qnext, unsigned* order_buf, int sms, int interval, int service, cudaStream_t s,
-                       int* launches, int lanes, int mpt, DoneRec* done = nullptr, unsigned by_count = 0);
+                       int* launches, int lanes, int mpt, DoneRec* done = nullptr, unsigned most = 0);
 
 }  // namespace ctraj

@@ -86,6 +86,7 @@ struct SweepLaunch {
   unsigned done_cap[CTRAJ_MAX_TABLES] = {};
   int outward = 0;                         // every configuration's force points away from the axis
   int threads = kPersistThreads;           // persistent: threads per CTA of k_sweep_persist
+  bool wide = false;                       // persistent: long queues take kSweepWideThreads instead
 };
 
 // The persistent sweep lens kernel of a force law; staged when every table
@@ -111,14 +112,11 @@ bool sweep_staged(const SweepLaunch& W) {
   return true;
 }
 
-// A sweep's linear pass with 512 lanes per CTA (the default) takes 768 for more queued molecules than kSweepWideRounds
-// rounds of 512: more warps per scheduler hide more of a step's latency, but a molecule's own steps take longer, which is
+// A sweep's linear pass without a set number of lanes takes 512 per CTA, and 768 for more queued molecules than
+// kSweepWideRounds rounds of 512 (SweepLaunch::wide): more warps per scheduler hide more of a step's latency, but a molecule's own steps take longer, which is
 // what a short queue waits for.  Rounds 3.3, 4.4, 6.7, 8.9, 22: 1.13, 1.08, 0.98, 0.97, 0.94 of the time with 512.  The
 // count is known on the device only, so both are launched and one returns.
 constexpr int kSweepWideThreads = 768, kSweepWideRounds = 6;
-bool sweep_wide(const SweepLaunch& W) {
-  return W.force == kForceStark2Lin && sweep_staged(W) && W.threads == kPersistThreads;
-}
 
 size_t sweep_persist_smem(const SweepLaunch& W, int threads) {
   int max_int = 0;
@@ -180,7 +178,7 @@ int sweep_enqueue(ctraj_context* c, const Plan& P, const RunDev& R, const SweepL
       ++launches;
       return cudaGetLastError();
     };
-    if (sweep_wide(W)) {
+    if (W.wide) {
       const unsigned few = unsigned(c->sm_count) * kPersistThreads * kSweepWideRounds;
       CT_CUDA(pass(W.threads, 0u, few));
       CT_CUDA(pass(kSweepWideThreads, few + 1u, 0xFFFFFFFFu));
@@ -433,7 +431,8 @@ extern "C" int ctraj_run_sweep(ctraj_context* c, const ctraj_sweep* sw, const ct
     L.n_smem = L.n_int <= (lin ? kMaxStagedLinear : kMaxStagedIntervals) ? L.n_int : 0;
   }
   W.chunks = sweep_chunks(c, sweep_step_estimate(e, a));
-  W.threads = W.force == kForceStark2Lin && sweep_staged(W) ? c->lens_threads : kPersistThreads;
+  W.wide = W.force == kForceStark2Lin && sweep_staged(W) && c->lens_threads == 0;
+  W.threads = W.force == kForceStark2Lin && sweep_staged(W) && c->lens_threads > 0 ? c->lens_threads : kPersistThreads;
 
   // what a captured graph depends on
   std::vector<char> key;
@@ -457,6 +456,7 @@ extern "C" int ctraj_run_sweep(ctraj_context* c, const ctraj_sweep* sw, const ct
   put(&W.force, sizeof W.force);
   put(&W.outward, sizeof W.outward);
   put(&W.threads, sizeof W.threads);
+  put(&W.wide, sizeof W.wide);
   const bool same = key == c->sweep_key;
   cudaStream_t s = c->stream;
   if (!same) {
@@ -511,7 +511,7 @@ extern "C" int ctraj_run_sweep(ctraj_context* c, const ctraj_sweep* sw, const ct
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   }
   if (W.persistent)
-    for (const int threads : {W.threads, sweep_wide(W) ? kSweepWideThreads : W.threads})
+    for (const int threads : {W.threads, W.wide ? kSweepWideThreads : W.threads})
       CT_CUDA(cudaFuncSetAttribute(sweep_persist_kernel(W.force, sweep_staged(W), threads),
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_persist_smem(W, threads))));
   CT_CUDA(cudaFuncSetAttribute(k_sweep_front<Mol32<false, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -5,7 +5,8 @@ launch that refills lanes and compacts the last molecules every
 ``lens_interval`` steps, or chunked launches), the length of the first lens
 chunk, the growth of later chunks and their maximum (how often molecules still
 inside a lens are compacted into full warps in chunked mode, which FP64 runs
-always use), the persistent pass's molecules per CTA (``lens_threads``) and
+always use), the persistent pass's molecules per CTA (``lens_threads``, 0: by
+the queue's length) and
 per thread (``lens_molecules``) and the steps between a warp's refills of
 its finished lanes (``lens_service``), the front kernel's grid (``front_waves``)
 and block size
@@ -28,7 +29,7 @@ import os
 from pathlib import Path
 
 DEFAULT = dict(chunk_first=64, chunk_growth=200, chunk_max=1024, front_waves=4, lens_mode=0, lens_interval=256,
-               front_threads=256, batch_group=4, lens_threads=512, lens_molecules=1, batch_lens_threads=1024,
+               front_threads=256, batch_group=4, lens_threads=0, lens_molecules=1, batch_lens_threads=0,
                lens_service=64)
 
 
@@ -43,6 +44,7 @@ def axes():
         if cm >= cf:
             lens.append(dict(lens_mode=1, chunk_first=cf, chunk_growth=g, chunk_max=cm))
     return [lens,
+            [dict(lens_threads=0, lens_molecules=1)] +
             [dict(lens_threads=lt, lens_molecules=m) for lt in (512, 768, 1024) for m in (1, 2)],
             [dict(lens_service=sv) for sv in (16, 32, 64, 128, 256)],
             [dict(lens_interval=iv) for iv in (64, 128, 256, 512, 1024)],
@@ -51,7 +53,7 @@ def axes():
 
 
 BATCH_GROUPS = (1, 2, 4, 8, 10, 16, 20, 32)
-BATCH_LENS_THREADS = (512, 768, 1024)
+BATCH_LENS_THREADS = (0, 512, 768, 1024)
 BATCH_SERVICE = (32, 64, 128, 256)
 
 

@@ -276,8 +276,14 @@ int ctraj_set_beamline(ctraj_context* ctx, const ctraj_element* elements,
  *                 at one molecule per thread that is 16, 24 or 32 warps per
  *                 SM within a register budget of 128, 80 or 64 per thread
  *                 (sweeps: linear Stark tables staged in shared memory;
- *                 others run 512).  At the default, linear tables take 768
- *                 or 1024 for queues of many rounds.            default 512
+ *                 others run 512).  0: by the lens queue's length.  Linear
+ *                 tables staged in shared memory then take 512 for a queue of
+ *                 up to 8 rounds of 512 per SM, 768 up to 32 and 1024 beyond
+ *                 (sweeps: 512 up to 6 rounds, 768 beyond), a single run the
+ *                 larger ones only where a 32nd of its molecules could fill
+ *                 such a queue: one most of whose molecules enter the lens
+ *                 may be faster with a set number.  Others take 512.
+ *                                                                  default 0
  *   lens_molecules molecules each thread of the persistent FP32 lens pass
  *                 steps in turn (1 or 2; with 2 the CTA has lens_threads / 2
  *                 threads, and each RK4 step has a second molecule's
@@ -288,9 +294,10 @@ int ctraj_set_beamline(ctraj_context* ctx, const ctraj_element* elements,
  *                 others run 512 x 1.
  *   batch_lens_threads lens_threads of the lens passes a batch group shares
  *                 (a group's pass is long enough that more warps per SM pay,
- *                 a single run's is set by its slowest molecule).  At the
- *                 default, linear tables take 512 or 768 for shorter queues.
- *                                                              default 1024 */
+ *                 a single run's is set by its slowest molecule).  0: linear
+ *                 tables as above, whatever share of the molecules enters the
+ *                 lens; others 512 up to one round and 1024 beyond.
+ *                                                                  default 0 */
 enum { CTRAJ_LENS_PERSISTENT = 0, CTRAJ_LENS_CHUNKED = 1 };
 
 #define CTRAJ_MAX_BATCH_GROUP 64
