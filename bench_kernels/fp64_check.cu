@@ -86,16 +86,28 @@ __global__ void k_sqrt32_check(unsigned long long* bad) {
   if (b) atomicAdd(bad, b);
 }
 
-// every y >= 0, infinity and a NaN, x = 0, at an edge of radius R and width 1 / inv_w
+// At an edge of radius R and width 1 / inv_w: every y >= 0, infinity and a NaN
+// with x = 0, then every squared radius t = x^2 + y^2: y is the root of t
+// rounded down and x the root of what is left, exact there, so that
+// fma(y, y, x x) rounds to t (from 2^-90 up, where what is left is a normal
+// number; one that is not t there is counted as well).
 __global__ void k_soft_test_check(float R, float inv_w, unsigned long long* bad) {
   unsigned long long b = 0;
   auto same = [](float p, float q) { return p == q || (isnan(p) && isnan(q)); };
-  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k <= 0x7f800001u; k += gridDim.x * blockDim.x) {
-    const float y = __uint_as_float(k);
+  auto differ = [&](float x, float y, float r2) {
     float ls, d, ls2, d2;
-    ctraj::soft_test(0.0f, y, R, inv_w, ls, d);
-    ctraj::soft_test_r2(__fmaf_rn(y, y, 0.0f), R, inv_w, ls2, d2);
-    b += same(ls, ls2) && same(d, d2) ? 0 : 1;
+    ctraj::soft_test(x, y, R, inv_w, ls, d);
+    ctraj::soft_test_r2(r2, R, inv_w, ls2, d2);
+    return same(ls, ls2) && same(d, d2) ? 0 : 1;
+  };
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k <= 0x7f800001u; k += gridDim.x * blockDim.x) {
+    const float v = __uint_as_float(k);
+    b += differ(0.0f, v, __fmaf_rn(v, v, 0.0f));
+    if (v < INFINITY) {
+      const float y = __fsqrt_rd(v), x = __fsqrt_rn(fmaxf(__fmaf_rn(-y, y, v), 0.0f));
+      const float t = __fmaf_rn(y, y, __fmul_rn(x, x));
+      b += differ(x, y, t) + (v >= 0x1p-90f && t != v ? 1 : 0);
+    }
   }
   if (b) atomicAdd(bad, b);
 }
