@@ -310,7 +310,7 @@ int enqueue_persistent(bool out, int mode, const Plan& P, const RunDev& R, int i
   // returns at once
   auto pass = [&](int lanes_, int mpt_, unsigned min_count, unsigned max_count) -> int {
     int kt = kPersistThreads, km = 1;
-    const PersistKernel k = persist_kernel(out, P.lf[i].force, mode, staged, lanes_, mpt_, &kt, &km);
+    const PersistKernel k = persist_kernel(out, P.lf[i].force, mode, staged, !done, lanes_, mpt_, &kt, &km);
     const size_t smem =
         (staged ? size_t(P.lf[i].n_int) * sizeof(float4) : 0) + size_t(kt) * size_t(km) * sizeof(SwapSlot);
     CT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));

@@ -246,14 +246,17 @@ int launch_chunk64(ctraj_context* c, bool out, const Plan& P, const RunDev& R, i
 // kernel returned.  512, 768 or 1024 lanes at one molecule per thread, and
 // for the hexapole Stark forms also at two, are compiled for the staged-table
 // plain and batch passes without per-molecule outputs (the throughput path);
-// every other pass and setting runs 512 threads x 1.
+// every other pass and setting runs 512 threads x 1, as does a plain one
+// without per-molecule outputs that ends its molecules itself (`ends`: no
+// records are given).
 struct DoneRec;  // kernels.cuh: a molecule's state after its last step, for k_lens_finish
 using PersistKernel = void (*)(const Plan, const RunDev, const int, const Queue, const Queue, const LensArgs,
                                const unsigned*, const int, const int, DoneRec*);
-PersistKernel persist_kernel(bool out, int force, int mode, bool staged, int lanes, int mpt, int* threads,
+PersistKernel persist_kernel(bool out, int force, int mode, bool staged, bool ends, int lanes, int mpt, int* threads,
                              int* used_mpt);
 template <int F>  // one force law's configurations (k_persist_<law>.cu)
-PersistKernel persist_kernel_for(bool out, int mode, bool staged, int lanes, int mpt, int* threads, int* used_mpt);
+PersistKernel persist_kernel_for(bool out, int mode, bool staged, bool ends, int lanes, int mpt, int* threads,
+                                 int* used_mpt);
 
 // k_lens_finish for a plain or batch pass (k_persist.cu).
 using FinishKernel = void (*)(const Plan, const RunDev, const int, const Queue, const Queue, const DoneRec*,

@@ -13,13 +13,13 @@ FinishKernel finish_kernel(int mode) {
   return mode == kModeBatch ? k_lens_finish<M, kModeBatch> : k_lens_finish<M, kModePlain>;
 }
 
-PersistKernel persist_kernel(bool out, int force, int mode, bool staged, int lanes, int mpt, int* threads,
+PersistKernel persist_kernel(bool out, int force, int mode, bool staged, bool ends, int lanes, int mpt, int* threads,
                              int* used_mpt) {
   switch (force) {
-    case kForceStark2: return persist_kernel_for<kForceStark2>(out, mode, staged, lanes, mpt, threads, used_mpt);
-    case kForceStark2Lin: return persist_kernel_for<kForceStark2Lin>(out, mode, staged, lanes, mpt, threads, used_mpt);
-    case kForceStark1: return persist_kernel_for<kForceStark1>(out, mode, staged, lanes, mpt, threads, used_mpt);
-    default: return persist_kernel_for<kForceRadial>(out, mode, staged, lanes, mpt, threads, used_mpt);
+    case kForceStark2: return persist_kernel_for<kForceStark2>(out, mode, staged, ends, lanes, mpt, threads, used_mpt);
+    case kForceStark2Lin: return persist_kernel_for<kForceStark2Lin>(out, mode, staged, ends, lanes, mpt, threads, used_mpt);
+    case kForceStark1: return persist_kernel_for<kForceStark1>(out, mode, staged, ends, lanes, mpt, threads, used_mpt);
+    default: return persist_kernel_for<kForceRadial>(out, mode, staged, ends, lanes, mpt, threads, used_mpt);
   }
 }
 

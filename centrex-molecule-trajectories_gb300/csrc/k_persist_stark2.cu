@@ -3,5 +3,5 @@
 #include "k_persist.cuh"
 
 namespace ctraj {
-template PersistKernel persist_kernel_for<kForceStark2>(bool, int, bool, int, int, int*, int*);
+template PersistKernel persist_kernel_for<kForceStark2>(bool, int, bool, bool, int, int, int*, int*);
 }  // namespace ctraj

@@ -994,13 +994,14 @@ __device__ __forceinline__ void lens_finish(const Plan& P, const RunDev& R, cons
   }
 }
 
-// lens_finish as a call of its own, for the passes whose ends are deferred: a
-// plain run ends in the pass no molecule (the allocation-free entry point all),
-// a sweep only the molecules beyond its end records, and inlined there
-// the end's code set the pass's register count (126 at 512 threads, spills
-// at 768 and 1024); called, it costs a stack frame on that cold path and the
-// pass fits 79 registers at 768 threads (lens pass of the bench's sweep 17.3
-// -> 16.1 ms at 768, 16.8 -> 15.8 ms at 1024 threads).
+// lens_finish as a call of its own, for the passes that end few molecules or
+// none beside a long loop of steps: a sweep ends in the pass only the molecules
+// beyond its end records, and inlined there the end's code set the pass's
+// register count (126 at 512 threads, spills at 768 and 1024); called, it costs
+// a stack frame on that cold path and the pass fits 79 registers at 768 threads
+// (lens pass of the bench's sweep 17.3 -> 16.1 ms at 768, 16.8 -> 15.8 ms at
+// 1024 threads).  A plain pass with kEnds (the allocation-free entry point)
+// ends all its molecules by it.
 template <class M, bool kOut, int kMode>
 __device__ __noinline__ void lens_finish_call(const Plan& P, const RunDev& R, const int li, const Queue& Qin,
                                               const Queue& Qnext, const bool fin, M& m, LensStep& st,
@@ -1053,7 +1054,10 @@ struct PersistSlot {
 // against; each slot s of a warp is finalised and refilled like a warp of
 // its own, and the compaction of phase B packs molecules into the lowest
 // threads' slots.  kMPT = 1 is the one-molecule pass.
-template <class M, bool kOut, int F, bool kStaged, int kMode, int kT = kPersistThreads, int kMPT = 1>
+// kEnds: a plain pass without per-molecule outputs ends its molecules itself
+// instead of deferring all ends.
+template <class M, bool kOut, int F, bool kStaged, int kMode, int kT = kPersistThreads, int kMPT = 1,
+          bool kEnds = false>
 __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, const int li, const Queue& Qin,
                                              const Queue& Qnext, const LensArgs& L, const unsigned* order,
                                              const int interval, const int service,
@@ -1296,15 +1300,20 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // finished (tallied, or queued at the next lens) and the slot becomes idle;
   // with `done`, only their state is written to their DoneRec and
   // k_lens_finish finishes them after the pass in full warps.
+  // kDeferAll: a batch pass, and a plain one but for kEnds, has a record for
+  // every molecule and no code for an end: beside it, even called out of line
+  // and never reached, the pass kept its molecule in memory for the call's sake
+  // (4e6 molecules, 2.96e6 of them through 1, 30 or 600 steps of a linear lens:
+  // 643, 764 and 3 024 us with the call, 562, 668 and 2 894 without).
+  constexpr bool kDeferAll = !kOut && (kMode == kModeBatch || (kMode == kModePlain && !kEnds));
   auto finalize = [&](PersistSlot<M>& x) {
     bool fin = x.phase == kLost || x.phase == kExit || x.phase == kBad;
     if (!__any_sync(kFull, fin)) return;
-    if constexpr (!kOut && (kMode == kModePlain || kMode == kModeBatch || kMode == kModeSweep)) {
-      // a batch pass always defers (its host always passes `done`); a plain
-      // pass or a sweep when given `done`, a sweep for the queue positions
-      // below done_cap (the records it has room for; the rest end here)
-      if (kMode == kModeBatch || done) {
-        const bool defer = fin && (kMode != kModeSweep || x.idx < done_cap);
+    if constexpr (!kOut && (kDeferAll || kMode == kModeSweep)) {
+      // a sweep defers for the queue positions below done_cap (the records it
+      // has room for; the rest end here)
+      if (kDeferAll || done) {
+        const bool defer = fin && (kDeferAll || x.idx < done_cap);
         if (defer) {
           int4* r = reinterpret_cast<int4*>(done + x.idx);
           r[0] = make_int4(__float_as_int(x.m.x), __float_as_int(x.m.y), __float_as_int(x.m.vx),
@@ -1317,16 +1326,16 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
                            int(unsigned(x.phase) | (x.flags & 3u) << 3 | unsigned(x.n0) << 5));
           x.phase = kIdle;
         }
-        if (kMode != kModeSweep) return;
+        if (kDeferAll) return;
         fin = fin && !defer;
         if (!__any_sync(kFull, fin)) return;
       }
     }
-    if constexpr (kMode == kModeSweep || (kMode == kModePlain && !kOut)) {
+    if constexpr (kMode == kModeSweep || (kEnds && !kOut)) {
       lens_finish_call<M, kOut, kMode>(P, R, li, Qin, Qnext, fin, x.m, x.st, x.phase, x.flags, x.idx, x.n0,
                                        x.fresh, x.cfg, S, acc);
       if (fin) x.phase = kIdle;
-    } else if constexpr (kOut || kMode != kModeBatch) {
+    } else if constexpr (!kDeferAll) {
       lens_finish<M, kOut, kMode>(P, R, li, Qin, Qnext, fin, x.m, x.st, x.phase, x.flags, x.idx, x.n0, x.fresh,
                                   x.cfg, S, acc);
       if (fin) x.phase = kIdle;
@@ -1497,7 +1506,8 @@ __device__ __forceinline__ void persist_flush(BlockTally& S, const RunDev& R, in
 // compile-time constant so that __launch_bounds__ gives the register budget
 // of that occupancy; kMPT molecules per thread (the swap area holds kT x kMPT
 // slots).
-template <class M, bool kOut, int F, bool kStaged, int kMode = kModePlain, int kT = kPersistThreads, int kMPT = 1>
+template <class M, bool kOut, int F, bool kStaged, int kMode = kModePlain, int kT = kPersistThreads, int kMPT = 1,
+          bool kEnds = false>
 __global__ void __launch_bounds__(kT, 1) k_lens_persist(const __grid_constant__ Plan P, const RunDev R,
                                                         const int li, const Queue Qin, const Queue Qnext,
                                                         const LensArgs L, const unsigned* order,
@@ -1514,9 +1524,9 @@ __global__ void __launch_bounds__(kT, 1) k_lens_persist(const __grid_constant__ 
   __syncthreads();
   PersistAcc acc;
   // a short queue spreads over all SMs through the interleaved first entries
-  persist_pass<M, kOut, F, kStaged, kMode, kT, kMPT>(P, R, li, Qin, Qnext, L, order, interval, service,
-                                                      gridDim.x * kT * kMPT, s_dyn, s_swap, s_wcount, S, acc,
-                                                      done);
+  persist_pass<M, kOut, F, kStaged, kMode, kT, kMPT, kEnds>(P, R, li, Qin, Qnext, L, order, interval, service,
+                                                             gridDim.x * kT * kMPT, s_dyn, s_swap, s_wcount, S, acc,
+                                                             done);
   // a batch's tallies went to its runs; deferred ends are tallied by k_lens_finish
   if (kMode != kModeBatch && !done) persist_flush(S, R, P.n_labels, acc);
 }
