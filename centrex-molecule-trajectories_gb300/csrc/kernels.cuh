@@ -1157,6 +1157,19 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // and pieces are loaded ahead (lens_step_ahead), a group with a missed piece
   // being done again; a warp that misses in more than half of its groups goes
   // on without.
+  // The quadratic form steps one at a time (lens_step_xy) where warps are full
+  // and the lens pushes outward, at half the bore: there the groups' packed
+  // lookups and the steps that the ended molecules take again cost more than the
+  // looks (2.96e6 molecules through 600 steps, table staged or not: 3 420 and
+  // 4 518 us in groups, 3 106 and 3 516 singly).
+  // In a focusing lens, with outputs beside a staged table (a margin, so a root,
+  // per step) and in sweeps the groups are the faster ones.
+  bool grouped = true;
+  if constexpr (F == kForceStark2 && !kSweep && !(kOut && kStaged)) {
+    const float s = __fmaf_rn(L.beta, 0.25f * L.bore2, -L.s0);
+    const unsigned i = min(__float2uint_rz(s), unsigned(L.n_int - 1));
+    grouped = !((kStaged ? s_tab : L.q)[i].x > 0.0f);
+  }
   auto run = [&](const int n_steps, const bool sparse) {
     bool any = false;
 #pragma unroll
@@ -1250,7 +1263,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           }
         }
       }
-      for (; k + kRunGroup <= n_steps; k += kRunGroup) {
+      for (; (grouped || sparse) && k + kRunGroup <= n_steps; k += kRunGroup) {
         if (k % 64 == 0) {
           any = false;
 #pragma unroll

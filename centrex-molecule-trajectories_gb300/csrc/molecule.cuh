@@ -911,13 +911,19 @@ struct Mol32 {
   }
   __device__ __forceinline__ void pair_end(const float dt, const float dt6, const float dt26, const StagePair& a,
                                           const StagePair& b, float& r2) {
-    const float2 p = pack2(x, y), v = pack2(vx, vy);
     const float2 sum = pack2(__fadd_rn(__fadd_rn(a.Lx.x, a.Lx.y), b.Lx.y), __fadd_rn(__fadd_rn(a.Ly.x, a.Ly.y), b.Ly.y));
-    const float2 dx = __ffma2_rn(pack2(dt26, dt26), sum, __fmul2_rn(pack2(dt, dt), v));
+    const float2 dx = __ffma2_rn(pack2(dt26, dt26), sum, __fmul2_rn(pack2(dt, dt), pack2(vx, vy)));
     const float2 ux = __fadd2_rn(a.Lx, b.Lx), uy = __fadd2_rn(a.Ly, b.Ly);  // (l1 + l4, l2 + l3)
     const float2 dv = __fmul2_rn(pack2(dt6, dt6), pack2(__fmaf_rn(2.0f, ux.y, ux.x), __fmaf_rn(2.0f, uy.y, uy.x)));
-    // s += inc with the rounding error carried in c (Fast2Sum: |s| >= |inc + c|
-    // holds because one step changes x and v by far less than their size)
+    add_carried(dx, dv);
+    ax = a.Lx.x;
+    ay = a.Ly.x;
+    r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
+  }
+  // s += inc with the rounding error carried in c (Fast2Sum: |s| >= |inc + c|
+  // holds because one step changes x and v by far less than their size)
+  __device__ __forceinline__ void add_carried(const float2 dx, const float2 dv) {
+    const float2 p = pack2(x, y), v = pack2(vx, vy);
     float2 cp = pack2(cx, cy), cv = pack2(cvx, cvy);
     const float2 d1 = __fadd2_rn(dx, cp), t1 = __fadd2_rn(p, d1);
     cp = __fadd2_rn(d1, neg2(__fadd2_rn(t1, neg2(p))));
@@ -931,9 +937,6 @@ struct Mol32 {
     cy = cp.y;
     cvx = cv.x;
     cvy = cv.y;
-    ax = a.Lx.x;
-    ay = a.Ly.x;
-    r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
   }
   template <int F, bool kStaged, bool kScaled, bool kFast>
   __device__ __forceinline__ void lens_step_pair(const LensArgs& L, const PairTable& T, const float dt, const float hdt,
@@ -978,6 +981,36 @@ struct Mol32 {
     pair_end(dt, dt6, dt26, a, b, r2);
   }
 
+  // The quadratic form's step with one force after the other and (x, y) packed
+  // throughout: the same values as lens_step_pair in fewer instructions (the
+  // interval by the conversion unit, which runs beside the others), but with its
+  // lookups on one chain.  For passes whose SMs are full (persist_pass).
+  template <bool kStaged, bool kScaled>
+  __device__ __forceinline__ void lens_step_xy(const LensArgs& L, const float4* tab, const float dt, const float hdt,
+                                               const float c2, const float dt6, const float dt26, float& r2,
+                                               const float beta, const float kappa) {
+    auto force = [&](const float2 p, const float q2) {
+      const float s = __fmaf_rn(beta, q2, -L.s0);
+      const unsigned i = min(__float2uint_rz(s), unsigned(L.n_int - 1));  // negative s and NaN -> 0
+      const float u = __fadd_rn(s, -__uint2float_rn(i));
+      const float4 q = kStaged ? tab[i] : __ldg(tab + i);
+      const float w = __fmaf_rn(u, __fmaf_rn(u, q.z, q.y), q.x), k = kScaled ? __fmul_rn(kappa, w) : w;
+      return __ffma2_rn(pack2(k, k), p, pack2(0.0f, -L.g));
+    };
+    auto radius2 = [](const float2 p) { return __fmaf_rn(p.y, p.y, __fmul_rn(p.x, p.x)); };
+    const float2 p = pack2(x, y), v = pack2(vx, vy), Hdt = pack2(hdt, hdt), Dt = pack2(dt, dt);
+    const float2 l1 = force(p, r2), k2 = __ffma2_rn(Hdt, l1, v), p2 = __ffma2_rn(pack2(c2, c2), v, p);
+    const float2 l2 = force(p2, radius2(p2)), k3 = __ffma2_rn(Hdt, l2, v), p3 = __ffma2_rn(Hdt, k2, p);
+    const float2 l3 = force(p3, radius2(p3)), p4 = __ffma2_rn(Dt, k3, p), l4 = force(p4, radius2(p4));
+    const float2 sum = __fadd2_rn(__fadd2_rn(l1, l2), l3);
+    const float2 dx = __ffma2_rn(pack2(dt26, dt26), sum, __fmul2_rn(Dt, v));
+    const float2 dv = __fmul2_rn(pack2(dt6, dt6), __ffma2_rn(pack2(2.0f, 2.0f), __fadd2_rn(l2, l3), __fadd2_rn(l1, l4)));
+    add_carried(dx, dv);
+    ax = l1.x;
+    ay = l1.y;
+    r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
+  }
+
   // One step looked at by itself; true when the molecule left the bore.  Without
   // kScaled the coordinate scale comes from L and kappa is folded into the table.
   template <int F, bool kStaged, bool kScaled = false>
@@ -985,8 +1018,11 @@ struct Mol32 {
                             const float dt6, const float dt26, const float4* s_tab, unsigned& flags,
                             const float beta = 0.0f, const float kappa = 1.0f) {
     float r2 = __fmaf_rn(y, y, __fmul_rn(x, x));
-    lens_step_pair<F, kStaged, kScaled, false>(L, pair_table<F>(L, kStaged ? s_tab : L.q), dt, hdt, c2, dt6, dt26, r2,
-                                               flags, kScaled ? beta : L.beta, kappa);
+    if constexpr (F == kForceStark2)
+      lens_step_xy<kStaged, kScaled>(L, kStaged ? s_tab : L.q, dt, hdt, c2, dt6, dt26, r2, kScaled ? beta : L.beta, kappa);
+    else
+      lens_step_pair<F, kStaged, kScaled, false>(L, pair_table<F>(L, kStaged ? s_tab : L.q), dt, hdt, c2, dt6, dt26, r2,
+                                                 flags, kScaled ? beta : L.beta, kappa);
     if (kOut) note(__fadd_rn(sqrtf(r2), -L.bore));
     return r2 > L.bore2;
   }
