@@ -890,6 +890,15 @@ constexpr unsigned kThinLanes = 256, kThinRounds = 3;  // persist_pass
 // many warps: 176-212 cycles per step at one warp per scheduler against 229-264,
 // but 39.6 against 33.6 cycles per warp and step at four.
 constexpr unsigned kSparseWarps = 4;
+// and the steps are short enough for the molecules that share a warp.  A piece is
+// missed where the coordinate's third difference is not small, which goes with
+// the cube of the step, and one lane's miss has the warp take a group again:
+// the pieces pay up to about 1.5 molecules per warp at 300 steps through the
+// lens, 6 at 600 and 25 at 1200.  600 steps, 27 molecules per warp: 150-173 us
+// with them, 119-126 without, and 1 per warp 79-90 with them.
+__device__ __forceinline__ bool ahead_pays(unsigned per_warp, unsigned steps) {
+  return float(steps) * float(steps) >= 240.0f * 240.0f * float(per_warp);
+}
 // Warps that n molecules of a CTA are spread over: four (one per scheduler) or
 // a multiple of it, as few as hold them.  Thin warps step faster than packed
 // ones: fewer bank conflicts, missed pieces and ends per warp.
@@ -1153,10 +1162,10 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // behind the record's last row, those of a group taken again stored again;
   // 1.25e8 molecules recorded every 50 steps: 10.4 ms, 15.3 with such groups
   // taken singly).
-  // sparse: few warps of the CTA have molecules, so the step's latency counts
-  // and pieces are loaded ahead (lens_step_ahead), a group with a missed piece
-  // being done again; a warp that misses in more than half of its groups goes
-  // on without.
+  // sparse: few warps of the CTA have molecules, so the step's latency counts.
+  // ahead: pieces are loaded ahead (lens_step_ahead), a group with a missed piece
+  // being done again; a warp of which a molecule misses in more than half of its
+  // groups goes on without.
   // The quadratic form steps one at a time (lens_step_xy) where warps are full
   // and the lens pushes outward, at half the bore: there the groups' packed
   // lookups and the steps that the ended molecules take again cost more than the
@@ -1170,7 +1179,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     const unsigned i = min(__float2uint_rz(s), unsigned(L.n_int - 1));
     grouped = !((kStaged ? s_tab : L.q)[i].x > 0.0f);
   }
-  auto run = [&](const int n_steps, const bool sparse) {
+  auto run = [&](const int n_steps, const bool sparse, const bool ahead) {
     bool any = false;
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) any = any || X[s].phase == kRun;
@@ -1234,7 +1243,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
       };
       const PairTable T = pair_table<F>(L, kStaged ? s_tab : L.q);
       if constexpr (F == kForceStark2Lin && kStaged && kMPT == 1) {
-        if (sparse) {
+        if (ahead) {
           PersistSlot<M>& x = X[0];
           const float b = kSweep ? x.beta : L.beta;
           LinAhead q;
@@ -1371,12 +1380,13 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     thin = gridDim.x / 8u;
   const unsigned dealt = static_entries - thin * (unsigned(kT) - kThinLanes);  // entries dealt out at first
   const unsigned share = blockIdx.x < n_in ? (n_in - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
-  unsigned busy = kT / 32u;  // warps with molecules
+  unsigned busy = kT / 32u, per_warp = 32u;  // warps with molecules, and how many each
+  const unsigned most_steps = *(volatile unsigned*)Qin.max_steps;
   if (short_queue) {
     busy = spread_warps<kT>(share);
-    const unsigned per = busy ? (share + busy - 1u) / busy : 0u;  // of the CTA's share, in order: a warp's live alike
-    const unsigned j = unsigned(warp) * per + unsigned(lane);
-    if (unsigned(lane) < per && j < share) take(X[0], j * gridDim.x + blockIdx.x);
+    per_warp = busy ? (share + busy - 1u) / busy : 0u;  // of the CTA's share, in order: a warp's live alike
+    const unsigned j = unsigned(warp) * per_warp + unsigned(lane);
+    if (unsigned(lane) < per_warp && j < share) take(X[0], j * gridDim.x + blockIdx.x);
   } else if (thin) {
     const bool in = blockIdx.x < thin;
     const unsigned j = in ? (unsigned(warp) * thin + blockIdx.x) * 32u + unsigned(lane)
@@ -1392,7 +1402,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // phase A (the further warps of a thin CTA wait at phase B's barrier)
   const bool further = blockIdx.x < thin && unsigned(warp) >= kThinLanes / 32u;
   for (bool exhausted = (dealt >= n_in && dealt > 0) || further; !exhausted;) {
-    run(service, false);
+    run(service, false, false);
     unsigned idle[kMPT], n_idle = 0;
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) {
@@ -1420,7 +1430,8 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
   // to the end of their molecules
   for (;;) {
     const bool last = kMPT == 1 && busy <= 4u;
-    run(last ? CTRAJ_MAX_LENS_STEPS : interval, busy <= kSparseWarps);
+    const bool sparse = busy <= kSparseWarps;
+    run(last ? CTRAJ_MAX_LENS_STEPS : interval, sparse, sparse && ahead_pays(per_warp, most_steps));
     unsigned held = 0;  // molecules this thread holds
 #pragma unroll
     for (int s = 0; s < kMPT; ++s) {
@@ -1448,6 +1459,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
     __syncthreads();
     if (total == 0) break;
     busy = kMPT == 1 ? spread_warps<kT>(total) : (total + 32 * kMPT - 1) / (32 * kMPT);
+    per_warp = (total + busy - 1u) / busy;
     if (busy < used) {
       unsigned r = base + excl;
 #pragma unroll
@@ -1469,7 +1481,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
       __syncthreads();
       // kMPT = 1: in order, evenly over `busy` warps; kMPT = 2: molecule q to slot
       // q % kMPT of thread q / kMPT, the lowest warps fill up
-      const unsigned per = kMPT == 1 ? (total + busy - 1u) / busy : 32u;
+      const unsigned per = kMPT == 1 ? per_warp : 32u;
 #pragma unroll
       for (int s = 0; s < kMPT; ++s) {
         PersistSlot<M>& x = X[s];

@@ -1,10 +1,15 @@
-"""The persistent FP32 lens pass takes the quadratic form's steps one at a time
-(full CTAs in a lens that pushes outward) or in groups.  Either gives the
-chunked pass's results."""
+"""The persistent FP32 lens pass picks the form of its steps by the table, the
+lens and how full its CTAs are: the quadratic form's one at a time (full CTAs in
+a lens that pushes outward) or in groups, the linear form's with table pieces
+loaded ahead or without (by the steps through the lens and the molecules per
+warp).  Every choice gives the chunked pass's results, and the runs' own ends
+those of the deferred ones."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+SMS_WARPS = 152 * 4  # warps that a short queue is spread over
 
 
 def _compiled(force, **step):
@@ -57,3 +62,14 @@ def test_quadratic_form(knots, low, n):
 
     force = ctraj.hexapole_force(V=10e3 if low else 30e3, R=17.5e-3, low_field_seeker=low, n_knots=knots)
     _equal_to_chunked(_compiled(force, dz=3e-3), n, 2.0)
+
+
+# 600, 300 and 240 steps through the lens: pieces ahead up to 6, 1 and 1 molecules per warp
+@pytest.mark.parametrize("dz,n", [(1e-3, 6 * SMS_WARPS), (1e-3, 6 * SMS_WARPS + 1), (1e-3, 30 * SMS_WARPS), (2e-3, SMS_WARPS),
+                                  (2e-3, SMS_WARPS + 1), (2.5e-3, 1), (2.6e-3, 1), (2e-4, 27 * SMS_WARPS)])
+@pytest.mark.parametrize("low", [False, True])
+def test_pieces_ahead(dz, n, low):
+    import ctraj
+
+    force = ctraj.hexapole_force(V=10e3 if low else 30e3, R=17.5e-3, low_field_seeker=low)
+    _equal_to_chunked(_compiled(force, dz=dz), n, 3.0)
