@@ -17,7 +17,8 @@
 //    pipes (a guessed interval is corrected against the knots, so the interval
 //    is the reference's).
 // A step in which a form is not sure of its rounding (2e-5 of the quotients and
-// roots), r = 0 or a lookup is outside the table is redone by Mol64::lens_step.
+// roots), r = 0 or a lookup is outside the table (with one lane per molecule: a
+// radial table) is redone by Mol64::lens_step.
 //
 // kQuad: four lanes per molecule, (stages 1 and 3 | stages 2 and 4) x (x | y):
 // stage 2 does not depend on stage 1, nor stage 4 on stage 3, so two force
@@ -56,21 +57,36 @@ struct Lens64 {
 };
 
 // a_r of lens_force64 at radius r; false when the plain path has to decide.
-template <int F>
-__device__ __forceinline__ bool accel64(const Lens64& L, const double2* rec, const double r, double& ar) {
+// kExtend: a spline's end pieces are extrapolated here, as PPoly does, and
+// `outside` is set.  With one lane per molecule the SMs are full, and a molecule
+// outside its table taking every step twice made the pass slower than
+// k_lens_chunk (74 000 molecules through 300 steps of a lens whose table begins
+// 2.5 mm off the axis: 14.2 ms there, 17.6 with the steps taken again, 8.8 so).
+// With four lanes taking them again still is the faster one (9.9 -> 5.6 ms), and
+// the steps inside the table are 1.4 % faster without the code for it.
+template <int F, bool kExtend>
+__device__ __forceinline__ bool accel64(const Lens64& L, const double2* rec, const double r, double& ar, bool& outside) {
   const double E = F == kForceRadial ? r : F == kForceStark1 ? __dmul_rn(L.alpha, r)
                                                              : __dmul_rn(L.alpha, __dmul_rn(r, r));
   // r is positive here, hence E is not negative; neither are the knots (records64)
-  if (less_pos(E, L.first) || !less_pos(E, L.last)) return false;
   int j = max(0, min(__float2int_rz((trunc_float(E) - L.x0) * L.inv_h), L.n - 1));
   double2 a, b;
-  for (;;) {
+  if (less_pos(E, L.first) || !less_pos(E, L.last)) {
+    if (F == kForceRadial || !kExtend) return false;
+    const bool below = less_pos(E, L.first);
+    j = below ? 0 : L.n - 1;
     a = rec[2 * j];
     b = rec[2 * j + 1];
-    const double next = rec[2 * j + 2].x;
-    if (less_pos(E, a.x)) --j;              // stops at j = 0: E >= first
-    else if (!less_pos(E, next)) ++j;       // and at n - 1: E < last
-    else break;
+    outside = outside || below || less_pos(L.last, E);
+  } else {
+    for (;;) {
+      a = rec[2 * j];
+      b = rec[2 * j + 1];
+      const double next = rec[2 * j + 2].x;
+      if (less_pos(E, a.x)) --j;              // stops at j = 0: E >= first
+      else if (!less_pos(E, next)) ++j;       // and at n - 1: E < last
+      else break;
+    }
   }
   const double s = dadd(E, -a.x);
   if (F == kForceRadial) {
@@ -147,10 +163,11 @@ __device__ __forceinline__ void advance_one64(Lane64& m, const Plan& P, const in
     bore_test(m, r, !isnan(r2), bore);
     if (k == chunk || !__any_sync(kFull, m.phase == kRun)) return;
     if (m.phase != kRun) continue;
+    bool outside = false;
     // l = the force at p, whose radius is r
     auto force = [&](const double (&p)[2], double (&l)[2]) {
       double ar = 0.0;
-      ok = ok && accel64<F>(L, rec, r, ar);
+      ok = ok && accel64<F, true>(L, rec, r, ar, outside);
       l[0] = div64(dmul(ar, p[0]), r, scale2(h, 1), sure);
       ok = ok && sure;
       l[1] = dadd(div64(dmul(ar, p[1]), r, scale2(h, 1), sure), -P.g);
@@ -211,6 +228,7 @@ __device__ __forceinline__ void advance_one64(Lane64& m, const Plan& P, const in
       }
       m.z = dadd(m.z, m.zinc);
       m.t = dadd(m.t, m.dt);
+      m.flags |= outside ? 1u : 0u;
     }
     ++m.n_done;
   }
@@ -230,7 +248,7 @@ __device__ __forceinline__ void advance_quad64(Lane64& m, const Plan& P, const i
   double X = m.x[0], V = m.v[0], zt = half ? m.t : m.z;
   const double zt_inc = half ? m.dt : m.zinc;
   for (int k = 0;; ++k) {
-    bool ok = true, sure;
+    bool ok = true, sure, outside = false;
     double h, r;
     auto radius = [&](const double p) {
       const double q = dmul(p, p), r2 = dadd(q, __shfl_xor_sync(kFull, q, 1));
@@ -240,7 +258,7 @@ __device__ __forceinline__ void advance_quad64(Lane64& m, const Plan& P, const i
     };
     auto force = [&](const double p) {
       double ar = 0.0;
-      ok = ok && accel64<F>(L, rec, r, ar);
+      ok = ok && accel64<F, false>(L, rec, r, ar, outside);
       const double l = dadd(div64(dmul(ar, p), r, scale2(h, 1), sure), g);
       ok = ok && sure;
       return l;
