@@ -90,7 +90,6 @@ __global__ void k_bm_check(const long long n, float* out) {
 
 }  // namespace
 
-// Returns 0 and the six largest errors above (out[6]) over n arguments.
 // out[0]: words w for which box_muller_pair differs from two box_muller calls
 // (w as U1 and as U2, in both components)
 namespace {
@@ -123,6 +122,7 @@ extern "C" int ctraj_peak_bm_pair_check(unsigned long long* mismatches) {
   return e == cudaSuccess ? 0 : -2;
 }
 
+// Returns 0 and the six largest errors above (out[6]) over n arguments.
 extern "C" int ctraj_peak_bm_check(long long n, float* out) {
   if (n < 1 || !out) return -1;
   float* d = nullptr;

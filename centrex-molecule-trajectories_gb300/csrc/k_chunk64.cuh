@@ -61,7 +61,7 @@ struct Lens64 {
 // `outside` is set.  With one lane per molecule the SMs are full, and a molecule
 // outside its table taking every step twice made the pass slower than
 // k_lens_chunk (74 000 molecules through 300 steps of a lens whose table begins
-// 2.5 mm off the axis: 14.2 ms there, 17.6 with the steps taken again, 8.8 so).
+// 2.4 mm off the axis: 14.2 ms there, 17.6 with the steps taken again, 8.8 so).
 // With four lanes taking them again still is the faster one (9.9 -> 5.6 ms), and
 // the steps inside the table are 1.4 % faster without the code for it.
 template <int F, bool kExtend>
