@@ -912,7 +912,9 @@ struct QuadShared {
   double last[2][8][8];                  // pair, (x, y, vx, vy, cx, cy, cvx, cvy), molecule
   int live[2][2];                        // pair, parity of the block: molecules left after its tests
 };
+// (the aligned form: the lanes meet first, some have left the last batch's end early)
 __device__ __forceinline__ void pair_sync(int pair) {
+  __syncwarp();
   asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
 }
 
