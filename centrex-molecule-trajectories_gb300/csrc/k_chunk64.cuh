@@ -29,7 +29,7 @@
 // molecule does the least work in total.
 //
 // Measured (lens beamline, GB300; Mol64::lens_step in 512-thread CTAs before):
-// 1e5 molecules 103 -> 15.0 ms (the slowest molecule's ~4 700 steps at 3.2 us;
+// 1e5 molecules 103 -> 15.0 ms (the longest stay's ~4 000 steps at 3.8 us;
 // 15.8 with the table's records read through L2 instead of shared memory),
 // 1e6 molecules 122 -> 21 ms, 3e6 130 -> 40 ms (1.1e9 steps/s).
 #pragma once

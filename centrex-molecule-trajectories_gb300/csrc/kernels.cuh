@@ -890,7 +890,7 @@ constexpr unsigned kThinLanes = 256, kThinRounds = 3;  // persist_pass
 // many warps: 176-212 cycles per step at one warp per scheduler against 229-264,
 // but 39.6 against 33.6 cycles per warp and step at four.
 constexpr unsigned kSparseWarps = 4;
-// and the steps are short enough for the molecules that share a warp.  A piece is
+// And only where the steps are short enough for the molecules that share a warp.  A piece is
 // missed where the coordinate's third difference is not small, which goes with
 // the cube of the step, and one lane's miss has the warp take a group again:
 // the pieces pay up to about 1.5 molecules per warp at 300 steps through the
@@ -1035,9 +1035,13 @@ struct __align__(16) DoneRec {
 static_assert(sizeof(DoneRec) == 64, "DoneRec is four 16-byte stores");
 
 // One CTA's share of a persistent pass over Qin.  The first static_entries
-// queue positions are dealt out interleaved across CTAs (entry (w * grid +
-// b) * 32 + lane to lane `lane` of warp w of CTA b); the rest are taken in
-// order by the lanes that become idle.  kModeSweep: molecules carry their
+// queue positions (none in a sweep) are dealt out interleaved across CTAs, entry
+// (w * grid + b) * 32 + lane to lane `lane` of warp w of CTA b; the rest are
+// taken in order by the lanes that become idle.  A queue shorter than that is
+// dealt out molecule by molecule, entry j * grid + b the j-th of CTA b, which
+// fills a few warps per scheduler evenly; and where some CTAs start thin (below)
+// they get the first entries and eight warps, the others the next ones as above,
+// fewer in all (`dealt`).  kModeSweep: molecules carry their
 // configuration (Queue::cfg), whose beta and kappa scale the unscaled table,
 // and tallies are also kept per configuration.  kModeBatch: molecules carry
 // their run (Queue::cfg) and every tally and stat goes to that run's slots
@@ -1194,7 +1198,7 @@ __device__ __forceinline__ void persist_pass(const Plan& P, const RunDev& R, con
           return;
         }
         const float4 sa = make_float4(x.m.x, x.m.y, x.m.vx, x.m.vy), sb = make_float4(x.m.cx, x.m.cy, x.m.cvx, x.m.cvy);
-        const int to_rec = x.to_rec;
+        [[maybe_unused]] const int to_rec = x.to_rec;
         const int how = advance();
         if (how == kGroupDone) {
           x.st.n_done += n;

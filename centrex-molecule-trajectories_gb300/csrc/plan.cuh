@@ -116,8 +116,8 @@ struct RunDev {
   const double* ics;  // (6, n) when injected
   ctraj_distribution xd, vd;
   float gap0f;         // FP32 first flight for drawn ICs: (float)(el[0].z0 - xd.z)
-  float xf[3], vf[6];  // xd.p (a disc: radius and z) and vd.p rounded to float: a conversion in the
-                       // kernel takes the FP64 pipe, per molecule where it is not hoisted
+  float xf[2], vf[6];  // the sigmas (a disc: xf[0] its radius) and vd.p rounded to float: a conversion
+                       // in the kernel takes the FP64 pipe, per molecule where it is not hoisted
   int32_t* out_label;
   double* out_final;   // (10, n)
   int32_t* out_rows;
@@ -214,8 +214,7 @@ struct SweepQueues {
 inline void round_distributions(RunDev& R) {
   const bool disc = R.xd.kind == CTRAJ_DIST_DISC_POSITION;
   R.xf[0] = float(disc ? R.xd.p[0] * 0.5 : R.xd.p[0]);
-  R.xf[1] = float(R.xd.p[1]);
-  R.xf[2] = float(R.xd.p[2]);
+  R.xf[1] = disc ? 0.0f : float(R.xd.p[1]);
   for (int k = 0; k < 6; ++k) R.vf[k] = float(R.vd.p[k]);
 }
 
