@@ -32,10 +32,10 @@
 namespace ctraj {
 
 // The exact-mode lens passes give a molecule four lanes up to this many
-// molecules in the queue: 1250 warps, two per scheduler of 152 SMs, take 75 x
-// 152 cycles a step of k_lens_chunk64, 313 warps of one lane per molecule 197 x
-// 64 (5 100 molecules, quads: 18.7 ms; 10 200, one lane while more than this are
-// left: 27 ms; 17 000: 40 ms).
+// molecules in the queue: 1250 warps, two or three per scheduler of 152 SMs, take
+// 87 x 152 cycles a step of k_lens_chunk64, 313 warps of one lane per molecule
+// 222 x 64 (5 100 molecules, quads: 18.7 ms; 10 200, one lane while more than this
+// are left: 27 ms; 17 000: 40 ms).
 constexpr unsigned kQuad64Max = 10000;
 
 __device__ __forceinline__ int hi_word(double a) { return __double2hiint(a); }

@@ -4,7 +4,8 @@
 //
 // Bound: the FP64 pipe (fp64.cuh: 64 cycles of a scheduler's pipe per warp
 // instruction, 19 per SM when all four pipes are busy).  Mol64::lens_step
-// issues ~480 FP64 instructions; the step here needs 197:
+// issues 421 FP64 instructions per warp and step, the step here 222 (counted by
+// ncu; all in the pipe, comparisons and conversions too):
 //  * square roots and quotients from fp64.cuh, the square root's reciprocal
 //    serving both components;
 //  * x + (dt v) / 2 and a + 2 b as one FMA (the scaling is exact, so the FMA
@@ -23,7 +24,7 @@
 // kQuad: four lanes per molecule, (stages 1 and 3 | stages 2 and 4) x (x | y):
 // stage 2 does not depend on stage 1, nor stage 4 on stage 3, so two force
 // evaluations follow one another instead of four, and each component has its
-// own lane: 75 FP64 instructions per step, at 4 x the warps.  A warp
+// own lane: 87 FP64 instructions per step, at 4 x the warps.  A warp
 // instruction costs the same for any number of lanes, so this is the shorter
 // way while the warps fit the schedulers (quad_max); beyond, one lane per
 // molecule does the least work in total.
